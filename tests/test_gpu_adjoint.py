@@ -200,3 +200,29 @@ def test_local_energy_vjp_central_difference():
     em = LocalEnergyGreens.apply(ga0 - h * da, gb0 - h * db, ham, trial, False).real.sum()
     fd = float(ep - em) / (2 * h)
     assert abs(ad - fd) < 1e-6 * max(1.0, abs(fd))
+
+
+@pytest.mark.parametrize("M,na,nb,X,W", [(33, 7, 1, 41, 5),  # odd rows (8-byte copies), clusters
+                                         (76, 10, 9, 50, 301),  # several walkers per CTA, a ragged last one
+                                         (200, 32, 31, 9, 3),  # one Cholesky vector per block, full shared memory
+                                         (256, 32, 32, 5, 2),  # single-buffered
+                                         (260, 8, 3, 7, 2),  # past M = 256: the scalar kernel
+                                         (8, 1, 1, 1, 1)])
+def test_local_energy_vjp_tile_edges(M, na, nb, X, W):
+    """The gradient at the edges of the kernel's tiles and buffers against torch autograd.  Sums of
+    products in FP64: the error of each is below (M + X N) eps of the absolute sums, 1e-10 relative."""
+    from types import SimpleNamespace
+
+    from ipie_b200.adjoint import LocalEnergyGreens
+
+    rng = np.random.default_rng(M)
+    c128 = lambda *s: torch.from_numpy(rng.normal(size=s) + 1j * rng.normal(size=s)).cuda()
+    real = lambda *s: torch.from_numpy(rng.normal(size=s)).cuda()
+    ham = SimpleNamespace(nchol=X, nbasis=M, ecore=1.5)
+    trial = SimpleNamespace(_rchola=real(X, na * M), _rcholb=real(X, nb * M), _rH1a=c128(na, M), _rH1b=c128(nb, M))
+    ga, gb, c = c128(W, na, M).requires_grad_(True), c128(W, nb, M).requires_grad_(True), c128(W)
+    e = LocalEnergyGreens.apply(ga, gb, ham, trial, False)
+    got = torch.autograd.grad((c * e).real.sum(), (ga, gb))
+    want = torch.autograd.grad((c * _torch_energy(ham, trial, ga, gb, False)).real.sum(), (ga, gb))
+    for a, b in zip(got, want):
+        assert rel(a, b) < 1e-10
