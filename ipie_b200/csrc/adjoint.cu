@@ -489,8 +489,9 @@ extern "C" int ipie_b200_local_energy_vjp(int rhf, const double* rchola, const d
   const bool alias = !rhf && nb == na && rcholb == rchola && ghalfb == ghalfa;
   const bool use_b = !rhf && nb > 0;
   // X_x = sum over the spins in the energy of L_s,x . G_s
-  cudaError_t e = launch_force_bias(rchola, ga, W, X, na * M, xv, 0, st, alias ? 2.0 : 1.0);
-  if (e == cudaSuccess && use_b && !alias) e = launch_force_bias(rcholb, gb, W, X, nb * M, xv, 1, st);
+  const bool two = use_b && !alias;
+  cudaError_t e = launch_force_bias(rchola, ga, na * M, two ? rcholb : nullptr, gb, nb * M, W, X, xv, st,
+                                    alias ? 2.0 : 1.0);
   if (e == cudaSuccess)
     e = launch_energy_vjp(rchola, ga, reinterpret_cast<const double2*>(rH1a), xv, eb, W, X, M, na, f1, fc, fx,
                           reinterpret_cast<double2*>(gbara), st);

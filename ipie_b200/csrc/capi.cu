@@ -42,9 +42,9 @@ int ipie_b200_construct_force_bias_batch_single_det(const double* rchola, const 
                                                     void* vbias, void* stream) {
   // Spin aliasing (rcholb == rchola, ghalfb == ghalfa, nb == na): one product, doubled (exactly t + t).
   const bool alias = nb == na && nb > 0 && rcholb == rchola && ghalfb == ghalfa;
-  cudaError_t e = launch_force_bias(rchola, CC2(ghalfa), W, X, na * M, C2(vbias), 0, ST(stream), alias ? 2.0 : 1.0);
-  if (e != cudaSuccess || nb == 0 || alias) return (int)e;
-  return (int)launch_force_bias(rcholb, CC2(ghalfb), W, X, nb * M, C2(vbias), 1, ST(stream));
+  const bool two = nb > 0 && !alias;
+  return (int)launch_force_bias(rchola, CC2(ghalfa), na * M, two ? rcholb : nullptr, CC2(ghalfb), nb * M, W, X,
+                                C2(vbias), ST(stream), alias ? 2.0 : 1.0);
 }
 
 int ipie_b200_field_shift(const void* vbias, const double* xi, const void* mf_shift, int W, int X, double sqrt_dt,
@@ -63,17 +63,13 @@ int ipie_b200_construct_vhs(const double* chol_packed, const int* idx_i, const i
 int ipie_b200_force_bias_complex(const double* r_re, const double* r_im, const void* ghalf, int W, int X, int K,
                                  void* out, int ld, int xoff, int accumulate, void* stream) {
   if (W <= 0 || X <= 0 || K <= 0 || ld < xoff + X || xoff < 0) return (int)cudaErrorInvalidValue;
-  cudaError_t e = launch_force_bias_c(r_re, CC2(ghalf), W, X, K, C2(out), ld, xoff, accumulate, 1.0, 0.0, ST(stream));
-  if (e != cudaSuccess) return (int)e;
-  return (int)launch_force_bias_c(r_im, CC2(ghalf), W, X, K, C2(out), ld, xoff, 1, 0.0, 1.0, ST(stream));
+  return (int)launch_force_bias_c(r_re, r_im, CC2(ghalf), W, X, K, C2(out), ld, xoff, accumulate, ST(stream));
 }
 
 int ipie_b200_construct_vhs_complex(const double* c_re, const double* c_im, int M, int F, const void* xshifted, int W,
                                     double sqrt_dt, void* vhs, void* stream) {
   if (M <= 0 || F <= 0 || W <= 0) return (int)cudaErrorInvalidValue;
-  cudaError_t e = launch_vhs_full(c_re, M, F, CC2(xshifted), W, sqrt_dt, C2(vhs), 0, ST(stream));
-  if (e != cudaSuccess) return (int)e;
-  return (int)launch_vhs_full(c_im, M, F, CC2(xshifted), W, sqrt_dt, C2(vhs), 1, ST(stream));
+  return (int)launch_vhs_full(c_re, c_im, M, F, CC2(xshifted), W, sqrt_dt, C2(vhs), ST(stream));
 }
 
 int ipie_b200_energy_complex(const void* ghalfa, const void* ghalfb, int W, int NMa, int NMb, const void* rh1a,
@@ -198,8 +194,8 @@ int ipie_b200_local_energy_single_det_batch(int rhf, const double* rchola, const
   double2* part = xv + (size_t)W * X;
   const bool alias = !rhf && nb == na && nb > 0 && rcholb == rchola && ghalfb == ghalfa;
   const int use_b = (!rhf && nb > 0 && !alias);
-  cudaError_t e = launch_force_bias(rchola, CC2(ghalfa), W, X, na * M, xv, 0, st, alias ? 2.0 : 1.0);
-  if (e == cudaSuccess && use_b) e = launch_force_bias(rcholb, CC2(ghalfb), W, X, nb * M, xv, 1, st);
+  cudaError_t e = launch_force_bias(rchola, CC2(ghalfa), na * M, use_b ? rcholb : nullptr, CC2(ghalfb), nb * M, W, X,
+                                    xv, st, alias ? 2.0 : 1.0);
   if (e != cudaSuccess) return (int)e;
   int rows_a = 0, rows_b = 0;
   e = launch_exchange(rchola, CC2(ghalfa), W, X, M, na, part, &rows_a, st);

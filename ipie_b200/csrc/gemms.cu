@@ -2,11 +2,12 @@
 // (DMMA): force bias, VHS assembly, one-body propagation, the Taylor series
 // of exp(VHS), and the fused exchange energy.
 #include "gemm_f64.cuh"
+#include "gemm_rc.cuh"
 #include "kernels.h"
 
 namespace ipie_b200 {
 
-// Large GEMMs (force bias, VHS, exchange): 128 x 64 CTA tile, 8 warps.
+// Exchange: 128 x 64 CTA tile, 8 warps.
 using CfgBig = TileCfg<128, 64, 16, 4, 2>;
 // Batched per-walker GEMMs: 64-row tile; the column tile follows 2N.
 using CfgW64 = TileCfg<64, 64, 16, 2, 4>;
@@ -14,32 +15,31 @@ using CfgW32 = TileCfg<64, 32, 16, 4, 2>;
 using CfgW16 = TileCfg<64, 16, 16, 4, 2>;
 
 // ---------------------------------------------------------------------------
-// Force bias: vbias[w][x] (+)= sum_k rchol[x][k] Ghalf[w][k]  (rchol real).
-// M = X rows, N = 2W interleaved (re, im) columns, K = N_s * M_basis.
+// Force bias: vbias[w][x] = scale sum_s sum_k rchol_s[x][k] Ghalf_s[w][k]  (rchol real), both spin
+// blocks in one launch.
 // ---------------------------------------------------------------------------
 struct EpiVbias {
   double2* v;
-  int X;
+  int ld, xoff;
   int accumulate;
   double scale;  // 2 for spin-aliased walkers: exactly t + t
-  __device__ __forceinline__ void operator()(int, int x, int col, double v0, double v1) const {
-    const size_t idx = (size_t)(col >> 1) * X + x;
-    double2 r = make_double2(scale * v0, scale * v1);
+  __device__ __forceinline__ void operator()(int x, int w, double2 c) const {
+    const size_t idx = (size_t)w * ld + xoff + x;
+    double2 r = cscale(c, scale);
     if (accumulate) r = cadd(r, v[idx]);
     v[idx] = r;
   }
 };
 
-cudaError_t launch_force_bias(const double* rchol, const double2* ghalf, int W, int X, int K, double2* vbias,
-                              int accumulate, cudaStream_t st, double scale) {
-  using C = CfgBig;
-  LoadRowK<C, C::BM> la{rchol, 0, K};
-  LoadWalkerCplx<C, C::BN> lb{reinterpret_cast<const double*>(ghalf), 2LL * K};
-  return launch_dmma_gemm<C>(X, 2 * W, K, 1, la, lb, EpiVbias{vbias, X, accumulate, scale}, st);
+cudaError_t launch_force_bias(const double* rchola, const double2* ghalfa, int Ka, const double* rcholb,
+                              const double2* ghalfb, int Kb, int W, int X, double2* vbias, cudaStream_t st,
+                              double scale) {
+  const RcSegment seg[2] = {{rchola, ghalfa, Ka, 0}, {rcholb, ghalfb, Kb, 0}};
+  return rc_gemm<true, false>(X, W, seg, rcholb != nullptr ? 2 : 1, EpiVbias{vbias, X, 0, 0, scale}, st);
 }
 
 // ---------------------------------------------------------------------------
-// VHS: VHS_packed[p][(w,c)] = sum_x L_packed[p][x] xshifted[x][(w,c)], scaled
+// VHS: VHS_packed[p][w] = sum_x L_packed[p][x] xshifted[x][w], scaled
 // by i sqrt(dt) and scattered to both triangles of the symmetric (W, M, M).
 // ---------------------------------------------------------------------------
 struct EpiVHS {
@@ -48,9 +48,8 @@ struct EpiVHS {
   const int* jj;
   int M;
   double sdt;
-  __device__ __forceinline__ void operator()(int, int p, int col, double v0, double v1) const {
-    const int w = col >> 1;
-    const double2 val = make_double2(-sdt * v1, sdt * v0);
+  __device__ __forceinline__ void operator()(int p, int w, double2 c) const {
+    const double2 val = make_double2(-sdt * c.y, sdt * c.x);
     const int i = ii[p], j = jj[p];
     double2* base = vhs + (size_t)w * M * M;
     base[(size_t)i * M + j] = val;
@@ -60,69 +59,37 @@ struct EpiVHS {
 
 cudaError_t launch_vhs(const double* chol_packed, const int* idx_i, const int* idx_j, int P, int X, int M,
                        const double2* xshifted, int W, double sqrt_dt, double2* vhs, cudaStream_t st) {
-  using C = CfgBig;
-  LoadRowK<C, C::BM> la{chol_packed, 0, X};
-  LoadRowR<C, C::BN> lb{reinterpret_cast<const double*>(xshifted), 0, 2LL * W};
-  return launch_dmma_gemm<C>(P, 2 * W, X, 1, la, lb, EpiVHS{vhs, idx_i, idx_j, M, sqrt_dt}, st);
+  const RcSegment seg{chol_packed, xshifted, X, 0};
+  return rc_gemm<false, false>(P, W, &seg, 1, EpiVHS{vhs, idx_i, idx_j, M, sqrt_dt}, st);
 }
 
 // ---------------------------------------------------------------------------
-// Complex-Cholesky pieces (ipie's GenericComplexChol), each built from real-operand
-// GEMMs of the same core: a complex operand R = R_re + i R_im enters as two launches,
-// the second scaled by i in the epilogue.
+// Complex-Cholesky pieces (ipie's GenericComplexChol): a complex operand R = R_re + i R_im enters
+// as two segments of one product, the second times i.
 //
-// Force bias / Coulomb vector: out[w][xoff + x] (+)= (sr + i si) sum_k R_part[x][k] Ghalf[w][k],
-// out rows of `ld` complex.
+// Force bias / Coulomb vector: out[w][xoff + x] (+)= sum_k R[x][k] Ghalf[w][k], out rows of `ld` complex.
 // ---------------------------------------------------------------------------
-struct EpiVbiasC {
-  double2* v;
-  int ld, xoff;
-  int accumulate;
-  double sr, si;
-  __device__ __forceinline__ void operator()(int, int x, int col, double v0, double v1) const {
-    const size_t idx = (size_t)(col >> 1) * ld + xoff + x;
-    double2 r = make_double2(sr * v0 - si * v1, sr * v1 + si * v0);
-    if (accumulate) r = cadd(r, v[idx]);
-    v[idx] = r;
-  }
-};
-
-cudaError_t launch_force_bias_c(const double* rpart, const double2* ghalf, int W, int X, int K, double2* out, int ld,
-                                int xoff, int accumulate, double sr, double si, cudaStream_t st) {
-  using C = CfgBig;
-  LoadRowK<C, C::BM> la{rpart, 0, K};
-  LoadWalkerCplx<C, C::BN> lb{reinterpret_cast<const double*>(ghalf), 2LL * K};
-  return launch_dmma_gemm<C>(X, 2 * W, K, 1, la, lb, EpiVbiasC{out, ld, xoff, accumulate, sr, si}, st);
+cudaError_t launch_force_bias_c(const double* r_re, const double* r_im, const double2* ghalf, int W, int X, int K,
+                                double2* out, int ld, int xoff, int accumulate, cudaStream_t st) {
+  const RcSegment seg[2] = {{r_re, ghalf, K, 0}, {r_im, ghalf, K, 1}};
+  return rc_gemm<true, true>(X, W, seg, 2, EpiVbias{out, ld, xoff, accumulate, 1.0}, st);
 }
 
 // VHS of a complex Cholesky: V_w = i sqrt(dt) C . xs_w with C = [A | B] (M*M, F) complex and
-// xs (F, W) complex, as two launches on C_re (mode 0: write) and C_im (mode 1: accumulate i x):
-//   C xs = (P0 - Q1) + i (P1 + Q0),  (P0, P1) = C_re (xs_re, xs_im),  (Q0, Q1) = C_im (xs_re, xs_im),
-//   V = i sqrt(dt) C xs:  Re V = -sdt (P1 + Q0),  Im V = sdt (P0 - Q1).
-// Rows p = i M + j of C map to V_w[i][j] directly (no symmetry).
+// xs (F, W) complex.  Rows p = i M + j of C map to V_w[i][j] directly (no symmetry).
 struct EpiVHSFull {
   double2* vhs;
   int M;
   double sdt;
-  int mode;
-  __device__ __forceinline__ void operator()(int, int p, int col, double v0, double v1) const {
-    const int w = col >> 1;
-    double2* dst = vhs + (size_t)w * M * M + p;
-    if (mode == 0) {
-      *dst = make_double2(-sdt * v1, sdt * v0);
-    } else {
-      const double2 o = *dst;
-      *dst = make_double2(o.x - sdt * v0, o.y - sdt * v1);
-    }
+  __device__ __forceinline__ void operator()(int p, int w, double2 c) const {
+    vhs[(size_t)w * M * M + p] = make_double2(-sdt * c.y, sdt * c.x);
   }
 };
 
-cudaError_t launch_vhs_full(const double* cpart, int M, int F, const double2* xshifted, int W, double sqrt_dt,
-                            double2* vhs, int mode, cudaStream_t st) {
-  using C = CfgBig;
-  LoadRowK<C, C::BM> la{cpart, 0, F};
-  LoadRowR<C, C::BN> lb{reinterpret_cast<const double*>(xshifted), 0, 2LL * W};
-  return launch_dmma_gemm<C>(M * M, 2 * W, F, 1, la, lb, EpiVHSFull{vhs, M, sqrt_dt, mode}, st);
+cudaError_t launch_vhs_full(const double* c_re, const double* c_im, int M, int F, const double2* xshifted, int W,
+                            double sqrt_dt, double2* vhs, cudaStream_t st) {
+  const RcSegment seg[2] = {{c_re, xshifted, F, 0}, {c_im, xshifted, F, 1}};
+  return rc_gemm<false, true>(M * M, W, seg, 2, EpiVHSFull{vhs, M, sqrt_dt}, st);
 }
 
 // Local energy of the complex-Cholesky form, one CTA per walker:

@@ -50,18 +50,20 @@ cudaError_t launch_energy_combine(int W, int X, int Ka, int Kb, const double2* g
                                   const double2* exx_part, int ntiles, double f1, double fc, double fx, double2* energy,
                                   unsigned* status, cudaStream_t st);
 
-cudaError_t launch_force_bias(const double* rchol, const double2* ghalf, int W, int X, int K, double2* vbias,
-                              int accumulate, cudaStream_t st, double scale = 1.0);
+// vbias = scale (rchola . ghalfa + rcholb . ghalfb); rcholb null: the first term alone
+cudaError_t launch_force_bias(const double* rchola, const double2* ghalfa, int Ka, const double* rcholb,
+                              const double2* ghalfb, int Kb, int W, int X, double2* vbias, cudaStream_t st,
+                              double scale = 1.0);
 cudaError_t launch_vhs(const double* chol_packed, const int* idx_i, const int* idx_j, int P, int X, int M,
                        const double2* xshifted, int W, double sqrt_dt, double2* vhs, cudaStream_t st);
 cudaError_t launch_one_body(const double* expH1, int cplx, const double2* phi_in, double2* phi_out, int W, int M, int N,
                             cudaStream_t st);
 cudaError_t launch_taylor(const double2* vhs, const double2* phi_in, double2* phi_out, double2* t0, double2* t1, int W,
                           int M, int N, int nmax, cudaStream_t st);
-cudaError_t launch_force_bias_c(const double* rpart, const double2* ghalf, int W, int X, int K, double2* out, int ld,
-                                int xoff, int accumulate, double sr, double si, cudaStream_t st);
-cudaError_t launch_vhs_full(const double* cpart, int M, int F, const double2* xshifted, int W, double sqrt_dt,
-                            double2* vhs, int mode, cudaStream_t st);
+cudaError_t launch_force_bias_c(const double* r_re, const double* r_im, const double2* ghalf, int W, int X, int K,
+                                double2* out, int ld, int xoff, int accumulate, cudaStream_t st);
+cudaError_t launch_vhs_full(const double* c_re, const double* c_im, int M, int F, const double2* xshifted, int W,
+                            double sqrt_dt, double2* vhs, cudaStream_t st);
 cudaError_t launch_scaled_row_sum(const double2* part, int rows, int W, double2 coef, double2* out, int accumulate,
                                   cudaStream_t st);
 cudaError_t launch_energy_complex(const double2* ga, const double2* gb, int W, int NMa, int NMb, const double2* rh1a,

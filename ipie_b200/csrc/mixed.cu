@@ -1355,10 +1355,8 @@ extern "C" int ipie_b200_local_energy_mixed(int rhf, const double* rchola, const
     }
   } else {
     // Coulomb vector in FP64 (DMMA): the Coulomb energy is the large, cancellation-free term
-    e = launch_force_bias(rchola, reinterpret_cast<const double2*>(ghalfa), W, X, na * M, xv, 0, st,
-                          alias ? 2.0 : 1.0);
-    if (e == cudaSuccess && use_b)
-      e = launch_force_bias(rcholb, reinterpret_cast<const double2*>(ghalfb), W, X, nb * M, xv, 1, st);
+    e = launch_force_bias(rchola, reinterpret_cast<const double2*>(ghalfa), na * M, use_b ? rcholb : nullptr,
+                          reinterpret_cast<const double2*>(ghalfb), nb * M, W, X, xv, st, alias ? 2.0 : 1.0);
     if (e != cudaSuccess) return (int)e;
   }
   // exchange: 3-pass FP16 tensor-core products (of G - G_T when the trial reference is given),
