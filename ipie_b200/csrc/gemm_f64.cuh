@@ -1,4 +1,5 @@
-// FP64 tensor-core GEMM core for the plain (FP64) walker step.
+// FP64 tensor-core GEMM core of the per-walker (batched) products of the plain (FP64) walker step: the
+// one-body factor and the Taylor terms outside the fused kernel's shapes.
 //
 // One CTA computes a BM x BN tile of C = sum_k A[m][k] B[k][n] with
 // warp-level DMMA (mma.sync m8n8k4 f64).  Operands are staged through shared
@@ -124,36 +125,6 @@ struct LoadCplxEmbed {
         r1[0] = v[i].y;
         r1[1] = v[i].x;
       }
-    }
-  }
-};
-
-// Walker-major complex operand read as real rows (w, c): element
-// (r = 2w + c, k) at p[w*ld + 2k + c] (ld in doubles).  Used for the
-// half-rotated Green's functions G[w][k] as the right operand of
-// rchol . G^T, so the output pair (n, n+1) is (re, im) of walker w.
-template <class Cfg, int ROWS>
-struct LoadWalkerCplx {
-  const double* p;
-  long long ld;
-  static constexpr int E = ROWS * Cfg::BK / Cfg::THREADS;
-  double v[E];
-  __device__ __forceinline__ void fetch(int b, int r0, int k0, int rows, int K) {
-    int w0 = r0 / 2;
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      int e = threadIdx.x + i * Cfg::THREADS;
-      int wl = e / (2 * Cfg::BK), rem = e % (2 * Cfg::BK);
-      int k = k0 + rem / 2, c = rem & 1, w = w0 + wl;
-      v[i] = (2 * w < rows && k < K) ? __ldg(p + (long long)w * ld + 2 * k + c) : 0.0;
-    }
-  }
-  __device__ __forceinline__ void commit(double* s) const {
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      int e = threadIdx.x + i * Cfg::THREADS;
-      int wl = e / (2 * Cfg::BK), rem = e % (2 * Cfg::BK);
-      s[(2 * wl + (rem & 1)) * Cfg::LDS + rem / 2] = v[i];
     }
   }
 };

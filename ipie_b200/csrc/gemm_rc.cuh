@@ -70,16 +70,19 @@ struct RcCfg {
   static_assert(BN % 8 == 0 && (LDBN & 7) == 2 && (LDBK & 7) == 4 && (LDA & 15) == 4, "conflict-free strides");
 };
 
-// WALKER_MAJOR: B[n][k]; else B[k][n].  TIMES_I: some segment has times_i.
-template <class C, bool WALKER_MAJOR, bool TIMES_I, class Epi>
-__global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int N, const __grid_constant__ RcOperands op, int S, Epi epi) {
-  extern __shared__ __align__(16) double rc_sm[];
+// One lane's accumulators: real and imaginary parts of rows 8 i + g, columns 8 j + 2 t + q of its warp tile.
+template <class C>
+struct RcAcc {
+  double re[C::FM][C::FN][2], im[C::FM][C::FN][2];
+};
+
+// Chunks c0 .. c1 - 1 of the tile at (m0, n0).  WALKER_MAJOR: B[n][k]; else B[k][n].  TIMES_I: some
+// segment has times_i.
+template <class C, bool WALKER_MAJOR, bool TIMES_I>
+__device__ __forceinline__ void rc_mainloop(int M, int N, int m0, int n0, const RcOperands& op, int c0, int c1,
+                                            double* rc_sm, RcAcc<C>& acc) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int wm0 = (warp / C::WARPS_N) * C::WTM, wn0 = (warp % C::WARPS_N) * C::WTN;
-  const int rank = (int)(blockIdx.x % S);
-  const int m0 = (int)blockIdx.y * C::BM, n0 = (int)(blockIdx.x / S) * C::BN;
-  const int c0 = (int)((long long)op.chunks * rank / S), c1 = (int)((long long)op.chunks * (rank + 1) / S);
-
   // next chunk to copy: its segment and first k
   int lseg = 0, lk = c0;
   while (lseg < op.nseg - 1 && lk >= (op.seg[lseg].K + kRcBK - 1) / kRcBK) {
@@ -137,11 +140,10 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int 
     cp_async_commit();  // an empty group past the end keeps one group per chunk
   };
 
-  double dr[C::FM][C::FN][2], di[C::FM][C::FN][2];
 #pragma unroll
   for (int i = 0; i < C::FM; ++i)
 #pragma unroll
-    for (int j = 0; j < C::FN; ++j) dr[i][j][0] = dr[i][j][1] = di[i][j][0] = di[i][j][1] = 0.0;
+    for (int j = 0; j < C::FN; ++j) acc.re[i][j][0] = acc.re[i][j][1] = acc.im[i][j][0] = acc.im[i][j][1] = 0.0;
 
   load(c0);
   load(c0 + 1);
@@ -169,8 +171,8 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int 
       for (int i = 0; i < C::FM; ++i)
 #pragma unroll
         for (int j = 0; j < C::FN; ++j) {
-          dmma884(dr[i][j], a[i], b[j].x);
-          dmma884(di[i][j], a[i], b[j].y);
+          dmma884(acc.re[i][j], a[i], b[j].x);
+          dmma884(acc.im[i][j], a[i], b[j].y);
         }
     }
     if (TIMES_I && (++ck) * kRcBK >= op.seg[cseg].K) {
@@ -178,6 +180,19 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int 
       cseg = min(cseg + 1, op.nseg - 1);
     }
   }
+}
+
+template <class C, bool WALKER_MAJOR, bool TIMES_I, class Epi>
+__global__ void __launch_bounds__(C::THREADS, C::OCC)
+    rc_gemm_kernel(int M, int N, const __grid_constant__ RcOperands op, int S, Epi epi) {
+  extern __shared__ __align__(16) double rc_sm[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wm0 = (warp / C::WARPS_N) * C::WTM, wn0 = (warp % C::WARPS_N) * C::WTN;
+  const int rank = (int)(blockIdx.x % S);
+  const int m0 = (int)blockIdx.y * C::BM, n0 = (int)(blockIdx.x / S) * C::BN;
+  RcAcc<C> acc;
+  rc_mainloop<C, WALKER_MAJOR, TIMES_I>(M, N, m0, n0, op, (int)((long long)op.chunks * rank / S),
+                                        (int)((long long)op.chunks * (rank + 1) / S), rc_sm, acc);
   if (S == 1) {
 #pragma unroll
     for (int i = 0; i < C::FM; ++i)
@@ -187,7 +202,7 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int 
         if (m >= M) continue;
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-          if (n + q < N) epi(m, n + q, make_double2(dr[i][j][q], di[i][j][q]));
+          if (n + q < N) epi(m, n + q, make_double2(acc.re[i][j][q], acc.im[i][j][q]));
       }
     return;
   }
@@ -201,8 +216,8 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC) rc_gemm_kernel(int M, int 
 #pragma unroll
     for (int j = 0; j < C::FN; ++j) {
       double2* d = sC + (wm0 + 8 * i + g) * C::LDC + wn0 + 8 * j + 2 * t;
-      d[0] = make_double2(dr[i][j][0], di[i][j][0]);
-      d[1] = make_double2(dr[i][j][1], di[i][j][1]);
+      d[0] = make_double2(acc.re[i][j][0], acc.im[i][j][0]);
+      d[1] = make_double2(acc.re[i][j][1], acc.im[i][j][1]);
     }
   cl.sync();
   const int rows = C::BM / S;  // BM and S are powers of two, S <= 8 <= BM

@@ -7,8 +7,6 @@
 
 namespace ipie_b200 {
 
-// Exchange: 128 x 64 CTA tile, 8 warps.
-using CfgBig = TileCfg<128, 64, 16, 4, 2>;
 // Batched per-walker GEMMs: 64-row tile; the column tile follows 2N.
 using CfgW64 = TileCfg<64, 64, 16, 2, 4>;
 using CfgW32 = TileCfg<64, 32, 16, 4, 2>;
@@ -238,136 +236,88 @@ cudaError_t launch_taylor(const double2* vhs, const double2* phi_in, double2* ph
 
 // ---------------------------------------------------------------------------
 // Fused exchange:  raw_w = sum_x sum_ij T_ij T_ji,  T = rchol_x (N x M) Ghalf_w^T.
-// GEMM rows (x, i) over X*NP (i padded to NP in {8,16,32}), columns
-// (w, j, c) over 2*W*NP, K = M.  The CTA tile holds complete NP x NP blocks
-// (x, w); the epilogue parks the tile in shared memory, forms the bilinear
-// trace per block and writes one partial per (x-tile, walker) -- T itself
-// never reaches global memory.
+// One product of the stacked rows (x, i) of rchol with the stacked columns (w, j) of Ghalf, K = M.
+// A tile takes as many whole vectors x and walkers w as fit its BM rows and BN columns, so no row or
+// column is spent on rounding N up (N = 10 in 16 x 16 blocks did 2.6 times the work); the tile shape
+// is the one of two that N fills better.  The epilogue parks T in shared memory and sums each
+// (x, w) block's products over unordered pairs (i, j) into one partial per (tile row, walker); T
+// never reaches global memory.  At 2 CTAs per SM one's epilogue runs under the other's products.
+// UHF, 640 walkers, M = 108, N = 15, X = 600, one spin: 1.99 -> 1.69 ms (37.3 GFLOP: 22
+// TFLOP/s, 25 with the padding of 15 to 120 / 8 rows); 512 walkers, M = 76, N = 10, X = 400: 0.78 -> 0.34 ms.
 // ---------------------------------------------------------------------------
-template <class C, int NP>
-struct LoadExchA {  // rows (x, i): rchol[x][i*M + m], zero for i >= N
-  const double* p;
-  int N, M;
-  static constexpr int E = C::BM * C::BK / C::THREADS;
-  double v[E];
-  __device__ __forceinline__ void fetch(int, int r0, int k0, int rows, int K) {
-#pragma unroll
-    for (int q = 0; q < E; ++q) {
-      int e = threadIdx.x + q * C::THREADS;
-      int r = r0 + e / C::BK, k = k0 + e % C::BK;
-      int x = r / NP, i = r % NP;
-      v[q] = (r < rows && i < N && k < K) ? __ldg(p + ((size_t)x * N + i) * M + k) : 0.0;
-    }
-  }
-  __device__ __forceinline__ void commit(double* s) const {
-#pragma unroll
-    for (int q = 0; q < E; ++q) {
-      int e = threadIdx.x + q * C::THREADS;
-      s[(e / C::BK) * C::LDS + e % C::BK] = v[q];
-    }
-  }
-};
+using ExWide = RcCfg<128, 32, 4, 2, 2>;
+using ExTall = RcCfg<96, 48, 4, 2, 2>;
 
-template <class C, int NP>
-struct LoadExchB {  // rows (w, j, c): Ghalf[w][j][m].c, zero for j >= N
-  const double* p;
-  int N, M;
-  static constexpr int E = C::BN * C::BK / C::THREADS;
-  double v[E];
-  __device__ __forceinline__ void fetch(int, int r0, int k0, int rows, int K) {
-#pragma unroll
-    for (int q = 0; q < E; ++q) {
-      int e = threadIdx.x + q * C::THREADS;
-      int pl = e / (2 * C::BK), rem = e % (2 * C::BK);
-      int k = k0 + rem / 2, c = rem & 1;
-      int pr = r0 / 2 + pl;  // (w, j) pair index
-      int w = pr / NP, j = pr % NP;
-      v[q] = (2 * pr < rows && j < N && k < K) ? __ldg(p + (((size_t)w * N + j) * M + k) * 2 + c) : 0.0;
-    }
-  }
-  __device__ __forceinline__ void commit(double* s) const {
-#pragma unroll
-    for (int q = 0; q < E; ++q) {
-      int e = threadIdx.x + q * C::THREADS;
-      int pl = e / (2 * C::BK), rem = e % (2 * C::BK);
-      s[(2 * pl + (rem & 1)) * C::LDS + rem / 2] = v[q];
-    }
-  }
-};
-
-template <class C, int NP>
-__global__ void __launch_bounds__(C::THREADS) exchange_kernel(const double* __restrict__ rchol,
-                                                              const double* __restrict__ ghalf, int W, int X, int M,
-                                                              int N, double2* __restrict__ part) {
-  extern __shared__ double smem[];
-  constexpr int XB = C::BM / NP;        // x values per tile
-  constexpr int WB = C::BN / (2 * NP);  // walkers per tile
-  const int m0 = blockIdx.y * C::BM, n0 = blockIdx.x * C::BN;
-  const int rows = X * NP, cols = 2 * W * NP;
-  LoadExchA<C, NP> la{rchol, N, M};
-  LoadExchB<C, NP> lb{ghalf, N, M};
-  Acc<C> acc;
-  dmma_mainloop<C>(0, m0, n0, rows, cols, M, la, lb, smem, acc);
-  // park the tile: sC[r][c] with row stride BN + 2
-  constexpr int LDC = C::BN + 2;
-  double* sC = smem;
+template <class C>
+__global__ void __launch_bounds__(C::THREADS, C::OCC)
+    exchange_kernel(const __grid_constant__ RcOperands op, int W, int X, int N, int XB, int WB,
+                    double2* __restrict__ part) {
+  extern __shared__ __align__(16) double rc_sm[];
+  constexpr int LDC = C::BN + 2;  // T_ij at stride LDC + 1 over i: odd, conflict-free
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wm0 = (warp / C::WARPS_N) * C::WTM, wn0 = (warp % C::WARPS_N) * C::WTN;
+  const int x0 = (int)blockIdx.y * XB, w0 = (int)blockIdx.x * WB;
+  RcAcc<C> acc;
+  rc_mainloop<C, true, false>(X * N, W * N, x0 * N, w0 * N, op, 0, op.chunks, rc_sm, acc);
+  cp_async_wait<0>();
+  __syncthreads();
+  double2* sT = reinterpret_cast<double2*>(rc_sm);
 #pragma unroll
   for (int i = 0; i < C::FM; ++i)
 #pragma unroll
     for (int j = 0; j < C::FN; ++j) {
-      int r = acc_row<C>(i), c = acc_col<C>(j);
-      sC[r * LDC + c] = acc.v[i][j][0];
-      sC[r * LDC + c + 1] = acc.v[i][j][1];
+      double2* d = sT + (wm0 + 8 * i + g) * LDC + wn0 + 8 * j + 2 * t;
+      d[0] = make_double2(acc.re[i][j][0], acc.im[i][j][0]);
+      d[1] = make_double2(acc.re[i][j][1], acc.im[i][j][1]);
     }
   __syncthreads();
-  // Each warp reduces (x_l, w_l) blocks: sum_{i,j<N} T_ij T_ji.
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = C::THREADS / 32;
-  __shared__ double2 wpart[XB * WB];
-  for (int blk = warp; blk < XB * WB; blk += nw) {
-    const int xl = blk / WB, wl = blk % WB;
+  // unordered pairs of {0..N-1} as (i, i + d mod N), d = 0 .. N/2: once each, except that d = N/2
+  // of an even N meets every pair twice
+  __shared__ double2 red[32];
+  const int nd = N / 2 + 1, xn = min(XB, X - x0), wn = min(WB, W - w0);
+  for (int wl = 0; wl < wn; ++wl) {
     double2 s = make_double2(0.0, 0.0);
-    const bool valid = (blockIdx.y * XB + xl) < X && (blockIdx.x * WB + wl) < W;
-    if (valid) {
-      for (int e = lane; e < N * N; e += 32) {
-        const int i = e / N, j = e % N;
-        const double* tij = sC + (xl * NP + i) * LDC + 2 * (wl * NP + j);
-        const double* tji = sC + (xl * NP + j) * LDC + 2 * (wl * NP + i);
-        s.x += tij[0] * tji[0] - tij[1] * tji[1];
-        s.y += tij[0] * tji[1] + tij[1] * tji[0];
-      }
+    for (int e = tid; e < xn * nd * N; e += C::THREADS) {
+      const int q = e / N, i = e - q * N, xl = q / nd, d = q - xl * nd;
+      const int j = i + d < N ? i + d : i + d - N;
+      const double2* blk = sT + xl * N * LDC + wl * N;
+      const double2 p = cmul(blk[i * LDC + j], blk[j * LDC + i]);
+      const double f = (d == 0 || 2 * d == N) ? 1.0 : 2.0;
+      s.x += f * p.x;
+      s.y += f * p.y;
     }
-    s = warp_sum2(s);
-    if (lane == 0) wpart[blk] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x < WB) {
-    const int w = blockIdx.x * WB + threadIdx.x;
-    if (w < W) {
-      double2 s = make_double2(0.0, 0.0);
-      for (int xl = 0; xl < XB; ++xl) s = cadd(s, wpart[xl * WB + threadIdx.x]);
-      part[(size_t)blockIdx.y * W + w] = s;
-    }
+    s = block_sum2(s, red);
+    if (tid == 0) part[(size_t)blockIdx.y * W + w0 + wl] = s;
   }
 }
 
-template <int NP>
-static cudaError_t exchange_np(const double* rchol, const double2* ghalf, int W, int X, int M, int N, double2* part,
-                               int* ntiles, cudaStream_t st) {
-  using C = CfgBig;  // 128 x 64
-  static_assert(C::BM % NP == 0 && C::BN % (2 * NP) == 0, "tile must hold whole blocks");
-  constexpr int XB = C::BM / NP, WB = C::BN / (2 * NP);
-  const int gx = (W + WB - 1) / WB, gy = (X + XB - 1) / XB;
-  *ntiles = gy;
-  if (part == nullptr) return cudaSuccess;
-  size_t smem = C::SMEM_DOUBLES * sizeof(double);
-  size_t need = (size_t)C::BM * (C::BN + 2) * sizeof(double);
-  if (need > smem) smem = need;
-  auto kern = exchange_kernel<C, NP>;
+template <class C>
+static cudaError_t exchange_cfg(const double* rchol, const double2* ghalf, int W, int X, int M, int N, double2* part,
+                                cudaStream_t st) {
+  const int XB = C::BM / N, WB = C::BN / N;
+  const size_t need = sizeof(double2) * C::BM * (C::BN + 2), smem = need > C::SMEM ? need : C::SMEM;
+  auto kern = exchange_kernel<C>;
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
-  kern<<<dim3(gx, gy), C::THREADS, smem, st>>>(rchol, reinterpret_cast<const double*>(ghalf), W, X, M, N, part);
+  RcOperands op = {};
+  op.seg[0] = RcSegment{rchol, ghalf, M, 0};
+  op.nseg = 1;
+  op.chunks = (M + kRcBK - 1) / kRcBK;
+  op.vec_a = M % 2 == 0 && reinterpret_cast<uintptr_t>(rchol) % 16 == 0;
+  op.vec_b = reinterpret_cast<uintptr_t>(ghalf) % 16 == 0;
+  kern<<<dim3((W + WB - 1) / WB, (X + XB - 1) / XB), C::THREADS, smem, st>>>(op, W, X, N, XB, WB, part);
   note_launch();
   return cudaGetLastError();
+}
+
+// The shape whose rows and columns N fills better, among those that need no more partial rows than
+// the N rounded up to 8, 16 or 32 takes in 128 (callers size fixed buffers by that count).
+static bool exchange_tall(int N) {
+  const int np = N <= 8 ? 8 : N <= 16 ? 16 : 32;
+  if (ExTall::BM / N < 128 / np) return false;
+  const int wide = (ExWide::BM / N * N) * (ExWide::BN / N * N) * (ExTall::BM * ExTall::BN);
+  const int tall = (ExTall::BM / N * N) * (ExTall::BN / N * N) * (ExWide::BM * ExWide::BN);
+  return tall > wide;
 }
 
 cudaError_t launch_exchange(const double* rchol, const double2* ghalf, int W, int X, int M, int N, double2* part,
@@ -376,10 +326,13 @@ cudaError_t launch_exchange(const double* rchol, const double2* ghalf, int W, in
     *ntiles = 0;
     return cudaSuccess;
   }
-  if (N <= 8) return exchange_np<8>(rchol, ghalf, W, X, M, N, part, ntiles, st);
-  if (N <= 16) return exchange_np<16>(rchol, ghalf, W, X, M, N, part, ntiles, st);
-  if (N <= 32) return exchange_np<32>(rchol, ghalf, W, X, M, N, part, ntiles, st);
-  return cudaErrorInvalidValue;
+  if (N > 32) return cudaErrorInvalidValue;
+  const bool tall = exchange_tall(N);
+  const int XB = (tall ? ExTall::BM : ExWide::BM) / N;
+  *ntiles = (X + XB - 1) / XB;
+  if (part == nullptr) return cudaSuccess;
+  return tall ? exchange_cfg<ExTall>(rchol, ghalf, W, X, M, N, part, st)
+              : exchange_cfg<ExWide>(rchol, ghalf, W, X, M, N, part, st);
 }
 
 }  // namespace ipie_b200
