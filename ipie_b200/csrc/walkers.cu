@@ -4,6 +4,7 @@
 //
 // One CTA owns one walker (both spin blocks) for the kernels that need the
 // walker's whole Slater matrix; its M x N orbitals live in shared memory.
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -239,106 +240,139 @@ cudaError_t launch_gf_overlap(const double2* phia, const double2* phib, int W, i
 // Field shift: from the force bias to the shifted fields of the VHS.
 //   xbar = -sqrt(dt) (i vbias - mf);  |xbar| > bound -> xbar/|xbar|
 //   xs = xi - xbar;  cmf = -sqrt(dt) sum_x xs mf;  cfb = sum_x xi xbar - xbar^2/2
-// One CTA per 32 walkers; the (X, W) transposed store goes through smem.
 // ---------------------------------------------------------------------------
-// FP16 head and remainder of the scaled x, both rounded to nearest (the 3-pass operand split)
-__device__ __forceinline__ void split_store_f16(__half* hi, __half* lo, size_t i, double x) {
-  const double y = x * kFieldScaleF16;
-  const __half h = __double2half(y);
-  hi[i] = h;
-  lo[i] = __double2half(y - (double)__half2float(h));
+// FP16 head and remainder of two neighbouring scaled x (the second when `two`), both rounded to nearest
+// (the 3-pass operand split); i even
+__device__ __forceinline__ void split_store_f16(__half* hi, __half* lo, size_t i, double x0, double x1, bool two) {
+  const double y0 = x0 * kFieldScaleF16, y1 = x1 * kFieldScaleF16;
+  const __half h0 = __double2half(y0), h1 = __double2half(y1);
+  const __half l0 = __double2half(y0 - (double)__half2float(h0)), l1 = __double2half(y1 - (double)__half2float(h1));
+  if (two) {
+    *reinterpret_cast<__half2*>(hi + i) = __halves2half2(h0, h1);
+    *reinterpret_cast<__half2*>(lo + i) = __halves2half2(l0, l1);
+  } else {
+    hi[i] = h0;
+    lo[i] = l0;
+  }
 }
 
-// xs_hi/xs_lo (optional): the shifted fields x kFieldScaleF16 as planar (W, 2, ldx) FP16
-// head/remainder, the right operand of the mixed-precision VHS product.
-__global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restrict__ vbias, const double* __restrict__ xi,
-                                                          const double2* __restrict__ mf, int W, int X, double sqrt_dt,
-                                                          double bound, double2* __restrict__ xshifted,
-                                                          double2* __restrict__ cmf, double2* __restrict__ cfb,
-                                                          __half* __restrict__ xs_hi, __half* __restrict__ xs_lo) {
-  __shared__ double2 tile[32][33];
-  const int ldx = f16_ld(X);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int w0 = blockIdx.x * 32;
-  double2 acc_mf[4], acc_fb[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) acc_mf[q] = acc_fb[q] = make_double2(0.0, 0.0);
-  for (int x0 = 0; x0 < X; x0 += 32) {
-    const int x = x0 + lane;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int wl = warp * 4 + q, w = w0 + wl;
-      double2 xs = make_double2(0.0, 0.0);
-      if (w < W && x < X) {
-        const double2 v = vbias[(size_t)w * X + x];
-        const double2 m = mf[x];
-        double2 xb = make_double2(-sqrt_dt * (-v.y - m.x), -sqrt_dt * (v.x - m.y));
-        const double a = cabs_(xb);
-        if (a > bound && a > 1e-13) xb = make_double2(xb.x / a, xb.y / a);
-        const double r = xi[(size_t)w * X + x];
-        xs = make_double2(r - xb.x, -xb.y);
-        if (xs_hi != nullptr) {
-          split_store_f16(xs_hi, xs_lo, ((size_t)w * 2) * ldx + x, xs.x);
-          split_store_f16(xs_hi, xs_lo, ((size_t)w * 2 + 1) * ldx + x, xs.y);
-        }
-        acc_mf[q] = cadd(acc_mf[q], cmul(xs, m));
-        double2 xb2 = cmul(xb, xb);
-        acc_fb[q] = cadd(acc_fb[q], make_double2(r * xb.x - 0.5 * xb2.x, r * xb.y - 0.5 * xb2.y));
-      }
-      tile[lane][wl] = xs;
-    }
-    __syncthreads();
-    // transposed store: row x, 32 consecutive walkers
-    if (xshifted != nullptr)
-      for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
-        const int xl = e / 32, wl = e % 32;
-        if (x0 + xl < X && w0 + wl < W) xshifted[(size_t)(x0 + xl) * W + w0 + wl] = tile[xl][wl];
-      }
-    __syncthreads();
+// One field: xbar bounded, the shifted field returned, cmf and cfb sums advanced.  |xbar| is compared
+// by its square first (hypot is 20 times the work and the bound is rarely met); near the bound the
+// comparison is hypot's.
+__device__ __forceinline__ double2 shift_one(double2 v, double2 m, double r, double sqrt_dt, double bound,
+                                             double near2, double2& acc_mf, double2& acc_fb) {
+  double2 xb = make_double2(-sqrt_dt * (-v.y - m.x), -sqrt_dt * (v.x - m.y));
+  if (xb.x * xb.x + xb.y * xb.y >= near2) {
+    const double a = cabs_(xb);
+    if (a > bound && a > 1e-13) xb = make_double2(xb.x / a, xb.y / a);
   }
+  const double2 xs = make_double2(r - xb.x, -xb.y);
+  acc_mf = cadd(acc_mf, cmul(xs, m));
+  const double2 xb2 = cmul(xb, xb);
+  acc_fb = cadd(acc_fb, make_double2(r * xb.x - 0.5 * xb2.x, r * xb.y - 0.5 * xb2.y));
+  return xs;
+}
+
+// With the (X, W) transposed copy (the FP64 VHS product's operand): a CTA takes 8 walkers, one per
+// warp, and a share of X in steps of 64; each step's 64 x 8 fields turn through shared memory so
+// that both sides move whole 128-byte lines.  The share is one of a cluster's S (the host's choice:
+// about four CTAs per SM, 64 fields or more each), whose partial sums are added through distributed
+// shared memory in rank order.  The first version, one CTA per 32 walkers over all of X, ran 2 to 32
+// CTAs: 84 -> 9 us at 640 walkers, X = 600; 37 -> 5.4 us at 256 walkers, X = 320; 14.7 -> 3.6 us at 64
+// walkers, X = 120.
+constexpr int kShiftWalkers = 8, kShiftStep = 64;
+__global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restrict__ vbias,
+                                                          const double* __restrict__ xi,
+                                                          const double2* __restrict__ mf, int W, int X, double sqrt_dt,
+                                                          double bound, double near2, int S,
+                                                          double2* __restrict__ xshifted, double2* __restrict__ cmf,
+                                                          double2* __restrict__ cfb, __half* __restrict__ xs_hi,
+                                                          __half* __restrict__ xs_lo) {
+  __shared__ double2 tile[2][kShiftStep][kShiftWalkers + 1];
+  __shared__ double2 part[kShiftWalkers][2];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int rank = (int)(blockIdx.x % S), w0 = (int)(blockIdx.x / S) * kShiftWalkers, w = w0 + wl;
+  const int steps = (X + kShiftStep - 1) / kShiftStep;
+  const int s0 = (int)((long long)steps * rank / S), s1 = (int)((long long)steps * (rank + 1) / S);
+  double2 acc_mf = make_double2(0.0, 0.0), acc_fb = make_double2(0.0, 0.0);
+  for (int s = s0; s < s1; ++s) {
+    double2(*buf)[kShiftWalkers + 1] = tile[s & 1];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    double2 a = warp_sum2(acc_mf[q]), b = warp_sum2(acc_fb[q]);
-    const int w = w0 + warp * 4 + q;
-    if (lane == 0 && w < W) {
-      cmf[w] = cscale(a, -sqrt_dt);
-      cfb[w] = b;
+    for (int h = 0; h < kShiftStep / 32; ++h) {
+      const int x = s * kShiftStep + 32 * h + lane;
+      if (w < W && x < X) {
+        const double2 xs = shift_one(vbias[(size_t)w * X + x], mf[x], xi[(size_t)w * X + x], sqrt_dt, bound, near2,
+                                     acc_mf, acc_fb);
+        buf[32 * h + lane][wl] = xs;
+        if (xs_hi != nullptr) {
+          const size_t o = (size_t)w * 2 * f16_ld(X) + x;
+          split_store_f16(xs_hi, xs_lo, o, xs.x, 0.0, false);
+          split_store_f16(xs_hi, xs_lo, o + f16_ld(X), xs.y, 0.0, false);
+        }
+      }
     }
+    __syncthreads();  // (the other buffer is rewritten only after the next step's barrier)
+#pragma unroll
+    for (int i = 0; i < kShiftStep * kShiftWalkers / 256; ++i) {
+      const int e = threadIdx.x + i * 256, xl = e / kShiftWalkers, c = e % kShiftWalkers;
+      const int x = s * kShiftStep + xl;
+      if (x < X && w0 + c < W) xshifted[(size_t)x * W + w0 + c] = buf[xl][c];
+    }
+  }
+  acc_mf = warp_sum2(acc_mf);
+  acc_fb = warp_sum2(acc_fb);
+  if (S > 1) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (lane == 0) {
+      part[wl][0] = acc_mf;
+      part[wl][1] = acc_fb;
+    }
+    cl.sync();
+    if (rank == 0 && lane == 0)
+      for (int q = 1; q < S; ++q) {
+        const double2* p = cl.map_shared_rank(&part[wl][0], q);
+        acc_mf = cadd(acc_mf, p[0]);
+        acc_fb = cadd(acc_fb, p[1]);
+      }
+    cl.sync();  // nobody leaves while its sums are being read
+  }
+  if (rank == 0 && lane == 0 && w < W) {
+    cmf[w] = cscale(acc_mf, -sqrt_dt);
+    cfb[w] = acc_fb;
   }
 }
 
 // The same shift without the (X, W) transposed copy: four warps per walker (two walkers per
-// block) walk its row of vbias / xi with coalesced loads, write the binary16 split and reduce cmf,
-// cfb with shuffles and shared memory (the mixed form, which needs no FP64 transposed fields; one
-// warp per walker left ~14 warps per SM, too few to cover the loads' latency).
+// block) walk its row of vbias / xi with coalesced loads, two neighbouring fields per lane, write the
+// binary16 split xs_hi / xs_lo (the fields x kFieldScaleF16 as planar (W, 2, ldx) head/remainder, the
+// right operand of the mixed VHS product) in pairs and reduce cmf, cfb with shuffles and shared
+// memory (one warp per walker left ~14 warps per SM, too few to cover the loads' latency).
 constexpr int kShiftWarps = 4;  // warps per walker
 __global__ void __launch_bounds__(256) field_shift_rows_kernel(const double2* __restrict__ vbias,
                                                                const double* __restrict__ xi,
                                                                const double2* __restrict__ mf, int W, int X,
-                                                               double sqrt_dt, double bound, double2* __restrict__ cmf,
-                                                               double2* __restrict__ cfb, __half* __restrict__ xs_hi,
-                                                               __half* __restrict__ xs_lo) {
+                                                               double sqrt_dt, double bound, double near2,
+                                                               double2* __restrict__ cmf, double2* __restrict__ cfb,
+                                                               __half* __restrict__ xs_hi, __half* __restrict__ xs_lo) {
   __shared__ double2 part[8][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % kShiftWarps;
   const int w = blockIdx.x * (8 / kShiftWarps) + warp / kShiftWarps;
   const bool live = w < W;
   const int ldx = f16_ld(X);
   double2 acc_mf = make_double2(0.0, 0.0), acc_fb = make_double2(0.0, 0.0);
-  for (int x = sub * 32 + lane; live && x < X; x += 32 * kShiftWarps) {
-    const double2 v = vbias[(size_t)w * X + x];
-    const double2 m = mf[x];
-    double2 xb = make_double2(-sqrt_dt * (-v.y - m.x), -sqrt_dt * (v.x - m.y));
-    const double a = cabs_(xb);
-    if (a > bound && a > 1e-13) xb = make_double2(xb.x / a, xb.y / a);
-    const double r = xi[(size_t)w * X + x];
-    const double2 xs = make_double2(r - xb.x, -xb.y);
+  for (int x = 2 * (sub * 32 + lane); live && x < X; x += 64 * kShiftWarps) {
+    const size_t e = (size_t)w * X + x;
+    const bool two = x + 1 < X;
+    double2 xs[2];
+    xs[0] = shift_one(vbias[e], mf[x], xi[e], sqrt_dt, bound, near2, acc_mf, acc_fb);
+    xs[1] = make_double2(0.0, 0.0);
+    if (two) xs[1] = shift_one(vbias[e + 1], mf[x + 1], xi[e + 1], sqrt_dt, bound, near2, acc_mf, acc_fb);
     if (xs_hi != nullptr) {
-      split_store_f16(xs_hi, xs_lo, ((size_t)w * 2) * ldx + x, xs.x);
-      split_store_f16(xs_hi, xs_lo, ((size_t)w * 2 + 1) * ldx + x, xs.y);
+      // rows of ldx (a multiple of 8) and even x: 4-byte stores; a pair's second half past X is padding
+      const size_t o = (size_t)w * 2 * ldx + x;
+      split_store_f16(xs_hi, xs_lo, o, xs[0].x, xs[1].x, two);
+      split_store_f16(xs_hi, xs_lo, o + ldx, xs[0].y, xs[1].y, two);
     }
-    acc_mf = cadd(acc_mf, cmul(xs, m));
-    const double2 xb2 = cmul(xb, xb);
-    acc_fb = cadd(acc_fb, make_double2(r * xb.x - 0.5 * xb2.x, r * xb.y - 0.5 * xb2.y));
   }
   acc_mf = warp_sum2(acc_mf);
   acc_fb = warp_sum2(acc_fb);
@@ -360,12 +394,31 @@ __global__ void __launch_bounds__(256) field_shift_rows_kernel(const double2* __
 cudaError_t launch_field_shift(const double2* vbias, const double* xi, const double2* mf, int W, int X, double sqrt_dt,
                                double bound, double2* xshifted, double2* cmf, double2* cfb, cudaStream_t st,
                                void* xs_hi, void* xs_lo) {
-  if (xshifted == nullptr)
-    field_shift_rows_kernel<<<(W + 1) / 2, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, cmf, cfb,
+  // below this square |xbar| is certainly not over the bound
+  const double near2 = bound > 0.0 ? bound * bound * (1.0 - 1e-12) : 0.0;
+  if (xshifted == nullptr) {
+    field_shift_rows_kernel<<<(W + 1) / 2, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, near2, cmf, cfb,
                                                          static_cast<__half*>(xs_hi), static_cast<__half*>(xs_lo));
-  else
-    field_shift_kernel<<<(W + 31) / 32, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, xshifted, cmf, cfb,
-                                                      static_cast<__half*>(xs_hi), static_cast<__half*>(xs_lo));
+    note_launch();
+    return cudaGetLastError();
+  }
+  const int groups = (W + kShiftWalkers - 1) / kShiftWalkers, steps = (X + kShiftStep - 1) / kShiftStep;
+  int S = 1;
+  while (S < 8 && 2 * S <= steps && groups * S < 4 * 148) S *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(groups * S));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)S;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, field_shift_kernel, vbias, xi, mf, W, X, sqrt_dt, bound, near2, S,
+                                           xshifted, cmf, cfb, static_cast<__half*>(xs_hi),
+                                           static_cast<__half*>(xs_lo));
+  if (e != cudaSuccess) return e;
   note_launch();
   return cudaGetLastError();
 }
