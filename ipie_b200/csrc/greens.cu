@@ -1,24 +1,7 @@
-// Green's function and overlap for spin blocks of N <= 32 electrons, one
-// 128-thread CTA per walker (42 KB of shared memory, four walkers per SM: two Ghalf columns per
-// lane and pass keep a thread within 128 registers; measured 12% faster than three):
-//
-//   O = phi^T psi*  (N x N): phi and psi* stream through shared memory in
-//       8-row chunks, a three-deep ring of cp.async copies issued two chunks
-//       ahead (one barrier per chunk); each thread accumulates a 2 x 4 block of
-//       O in registers;
-//   X = (P O)^-1 by Gauss-Jordan elimination in place in shared memory with
-//       partial pivoting on |.| (warp 0 picks the pivot, all threads update) --
-//       the pivots are those of the LU factorisation, so
-//       log|det O| = sum log|pivot_k|, phase = (-1)^swaps prod pivot_k / |pivot_k|
-//       (one pivot per lane of warp 0, reduced with shuffles);
-//   Ghalf[i, m] = sum_r X[i, r] phi[m, perm(r)] (= (O^-1 phi^T)[i, m]): a
-//       register-tiled product -- warp w takes rows 8w..8w+7, lane l the
-//       columns l + 32q (q < 2, so 64 columns per pass), phi staged in shared
-//       memory 4 permuted columns at a time, transposed, through a four-deep
-//       cp.async ring issued three steps ahead -- instead of one latency-bound
-//       pair of triangular solves per column.
+// Green's function, overlap and reorthogonalisation for spin blocks of N <= 32 electrons: one CTA of
+// 96 or 128 threads per walker, four per SM, the products on the f64 tensor cores.
 // ovlp_w = prod_s phase_s * exp(sum_s log|det O_s| - log_shift_w).
-// Same contract as gf_overlap_kernel (walkers.cu), which keeps N > 32.
+// Same contracts as gf_overlap_kernel and reortho_kernel (walkers.cu), which keep N > 32.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -107,204 +90,319 @@ __device__ void o_product(const double2* __restrict__ phi, const double2* __rest
     for (int q = 0; q < 4; ++q) sO[ti + 16 * a][tj + 8 * q] = acc[a][q];
 }
 
-// O = phi^T psi* for one spin block into sO; then its inverse (of the row-permuted O) in place,
-// the row order in sPerm and log|det|, phase from the pivots.
-__device__ SpinDet32 invert_block(const double2* __restrict__ phi, const double2* __restrict__ psic, int M, int N,
-                                  double2 (*sO)[kNP], double2* sStage, int* sPerm, double2* sPiv, double2* red,
-                                  unsigned* status) {
-  const int tid = threadIdx.x;
-  o_product<false>(phi, psic, M, N, sO, sStage);
-  if (tid < 32) sPerm[tid] = tid;
-  __syncthreads();
-  // ---- Gauss-Jordan with partial pivoting, in place: after step k row k holds the k-th row of
-  // the reduced inverse and column k the multipliers.  Two barriers per step: warp 0 picks the
-  // pivot (one redux.sync on a 32-bit key: the float bits of |a|^2 above the row index, so a
-  // pivot within ~2e-6 of the largest, the lowest row on ties), swaps it into row k and scales
-  // that row by 1/p (1/p = conj(p) / |p|^2, one reciprocal); then all threads update the rest with
-  // the scaled row (thread: column tid % 32, rows tid / 32 + 4r), the owners of column k-1 first
-  // applying that column's -1/p_{k-1} to their rows (deferred from step k-1: it commutes with the
-  // row swap and the row scaling; warp 0 applies it to row k's entry with the row scaling), which
-  // keeps a load-multiply-store off warp 0's serial chain.
-  int swaps = 0;
-  const int uj = tid & 31, ui = tid >> 5;
-  double2 pinv_prev = make_double2(0.0, 0.0);
-  for (int k = 0; k < N; ++k) {
-    if (tid < 32) {
-      unsigned key = 0u;
-      if (tid >= k && tid < N)
-        key = (__float_as_uint((float)cabs2(sO[tid][k])) & ~31u) | (unsigned)(31 - tid);
-      const int bi = 31 - (int)(__reduce_max_sync(0xffffffffu, key) & 31u);
-      // swap rows k and bi (all N columns) and the row order
-      if (bi != k && tid < N) {
-        const double2 t = sO[k][tid];
-        sO[k][tid] = sO[bi][tid];
-        sO[bi][tid] = t;
-      }
-      if (bi != k && tid == 0) {
-        const int t = sPerm[k];
-        sPerm[k] = sPerm[bi];
-        sPerm[bi] = t;
-      }
-      if (bi != k) ++swaps;  // warp-uniform: every lane of warp 0 counts
-      __syncwarp();
-      // row k x 1/p, a_kk = 1/p
-      const double2 pv = sO[k][k];
-      const double rn = __drcp_rn(pv.x * pv.x + pv.y * pv.y);
-      const double2 pinv = make_double2(pv.x * rn, -pv.y * rn);
-      if (tid < N && tid != k) {
-        double2 v = cmul(sO[k][tid], pinv);
-        // row k's entry of column k-1 also takes that column's deferred -1/p_{k-1}
-        if (tid == k - 1) v = cmul(v, make_double2(-pinv_prev.x, -pinv_prev.y));
-        sO[k][tid] = v;
-      }
-      if (tid == 0) {
-        if (pv.x == 0.0 && pv.y == 0.0) flag(status, STATUS_SINGULAR);
-        sPiv[k] = pv;
-        sO[k][k] = pinv;
-        red[5] = pinv;
+// ---------------------------------------------------------------------------------------------
+// The Green's function on the f64 tensor cores, N padded to NT tiles of 8.  Per walker and spin:
+//   O = phi^T psi*: chunks of 8 rows of phi and psi* through a three-deep cp.async ring; warp w
+//       owns row tile w of O (NT = 1: a quarter of the rows m, NT = 2: one of the four tiles).
+//   O^-1 by Gauss-Jordan elimination in place, partial pivoting on |.|, in panels of 8 columns: one
+//       warp factors the panel with a row per lane and the 8 columns in registers (the pivot by one
+//       redux.sync on the float bits of |a|^2 above the row index, its row by shuffles; pivots stay
+//       in their rows), then all warps apply it to the other columns as one rank-8 MMA update
+//         A[:, J] <- A[:, J] (pivot rows zeroed) + panel' A[pivot rows, J].
+//       So a column costs no barrier and a panel three, where the column by column form took two
+//       per column.
+//   With p_k the pivot row of column k the stored array B holds O^-1[k, p_j] = B[p_k, j].
+//   Ghalf[i, m] = sum_c O^-1[i, c] phi[m, c]: warp w keeps its rows of O^-1 as MMA fragments in
+//       registers (gathered through p once) while chunks of 16 rows of phi pass through the ring.
+//       The eight rows m of a tile are dealt to the MMA's columns as 0 4 1 5 2 6 3 7, so that four
+//       lanes store four neighbouring entries of Ghalf; rows of an odd stride keep the fragment
+//       loads free of bank conflicts.
+// The floor is the f64 tensor pipe's time for the two products (28k cycles per SM and walker at
+// M = 200, N = 32).  2048 walkers, M = 200, N = 32: 535 -> 354 us; 512, M = 76, N = 10: 46 -> 19 us; 777, M =
+// 149, N = 23 + 17: 280 -> 175 us (against DFMA products and the column by column elimination).
+template <int NT>
+struct GfShape {
+  static constexpr int WARPS = NT == 3 ? 3 : 4, THREADS = 32 * WARPS, NP = 8 * NT;
+  static constexpr int LDO = NP + 4;   // O (MMA left operand: 4 mod 8)
+  static constexpr int LDP = 12;       // panel
+  static constexpr int LDC = NP + 2;   // chunks of the O product (2 mod 8)
+  static constexpr int LDG = NP + 1;   // chunks of the Ghalf product (odd)
+  static constexpr int GM = 16;        // rows of phi per Ghalf chunk
+  static constexpr int RING = 3;
+  static constexpr int OSTAGE = 2 * kChunk * LDC, GSTAGE = GM * LDG;
+  static constexpr int STAGE = RING * (OSTAGE > GSTAGE ? OSTAGE : GSTAGE);
+  static constexpr int MW = WARPS / NT;  // warps sharing a row tile in the Ghalf product
+  static_assert(STAGE >= 4 * 64, "partial sums of the split O product fit the ring");
+};
+
+template <int NT>
+struct GfShared {
+  using S = GfShape<NT>;
+  double2 O[S::NP * S::LDO];
+  double2 P[S::NP * S::LDP];
+  double2 stage[S::STAGE];
+  double2 piv[32];
+  double2 red[4];
+  int perm[32], inv[32];
+  unsigned used;
+};
+
+template <int NT>
+__device__ __forceinline__ void gf_overlap_tiles(const double2* __restrict__ phi, const double2* __restrict__ psic,
+                                                 int M, int N, GfShared<NT>& sm) {
+  using S = GfShape<NT>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nch = (M + kChunk - 1) / kChunk;
+  auto issue = [&](int ch) {
+    if (ch < nch) {
+      double2* st = sm.stage + (ch % S::RING) * S::OSTAGE;
+      for (int e = tid; e < kChunk * S::NP; e += S::THREADS) {
+        const int r = e / S::NP, c = e % S::NP, m = ch * kChunk + r;
+        const bool in = m < M && c < N;
+        const size_t off = in ? (size_t)m * N + c : 0;
+        cp_async16(st + r * S::LDC + c, phi + off, in ? 16 : 0);
+        cp_async16(st + (kChunk + r) * S::LDC + c, psic + off, in ? 16 : 0);
       }
     }
+    cp_async_commit();  // (an empty group past the end keeps the group count per chunk)
+  };
+  constexpr int CT = NT >= 3 ? NT : 1;  // column tiles per warp
+  const int rt = NT >= 3 ? warp : NT == 2 ? (warp & 1) : 0, ct0 = NT == 2 ? (warp >> 1) : 0;
+  double re[CT][2], im[CT][2];
+#pragma unroll
+  for (int j = 0; j < CT; ++j) re[j][0] = re[j][1] = im[j][0] = im[j][1] = 0.0;
+  issue(0);
+  issue(1);
+  for (int ch = 0; ch < nch; ++ch) {
+    cp_async_wait<1>();
     __syncthreads();
-    // a_ij -= a_ik (a_kj / a_kk) for i, j != k (the scaled row k; column k is only read here).
-    // All of a thread's loads first: interleaved, each row's store could alias (for the compiler)
-    // the next row's loads, which made the eight rows a serial chain.
-    const double2 pk = red[5];
-    if (uj < N && uj != k) {
-      const double2 akj = sO[k][uj];
-      double2 a[8], f[8];
+    issue(ch + 2);
+    // NT = 1: the warps take turns at the 4-row steps
+    if (NT == 1 && (ch >> 1) % 2 != (warp >> 1)) continue;
+    const double2* a = sm.stage + (ch % S::RING) * S::OSTAGE + t * S::LDC + rt * 8 + g;
+    const double2* b = sm.stage + (ch % S::RING) * S::OSTAGE + (kChunk + t) * S::LDC + ct0 * 8 + g;
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = ui + 4 * r;
-        a[r] = sO[i][uj];
-        f[r] = sO[i][k];
-      }
-      if (uj == k - 1) {
-        // column k-1 x -1/p_{k-1} for rows other than k-1 (row k's entry: warp 0 above)
-        const double2 m = make_double2(-pinv_prev.x, -pinv_prev.y);
+    for (int kk = 0; kk < kChunk; kk += 4) {
+      if (NT == 1 && (kk >> 2) != (warp & 1)) continue;
+      const double2 av = a[kk * S::LDC];
 #pragma unroll
-        for (int r = 0; r < 8; ++r)
-          if (ui + 4 * r != k - 1) a[r] = cmul(a[r], m);
-      }
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = ui + 4 * r;
-        if (i < N && i != k) sO[i][uj] = csub(a[r], cmul(f[r], akj));
+      for (int j = 0; j < CT; ++j) {
+        const double2 bv = b[kk * S::LDC + 8 * j];
+        dmma884(re[j], av.x, bv.x);
+        dmma884(im[j], av.x, bv.y);
+        dmma884(re[j], -av.y, bv.y);
+        dmma884(im[j], av.y, bv.x);
       }
     }
-    pinv_prev = pk;
+  }
+  cp_async_wait<0>();
+  if (NT == 1) {
+    __syncthreads();  // the ring is free: the four partial tiles
+    double2* part = sm.stage + warp * 64 + g * 8 + 2 * t;
+    part[0] = make_double2(re[0][0], im[0][0]);
+    part[1] = make_double2(re[0][1], im[0][1]);
     __syncthreads();
-  }
-  // column N-1 x -1/p_{N-1} (rows other than N-1)
-  if (N > 0 && uj == N - 1) {
-    const double2 m = make_double2(-pinv_prev.x, -pinv_prev.y);
+    if (tid < 64) {
+      double2 v = sm.stage[tid];
+      for (int q = 1; q < 4; ++q) v = cadd(v, sm.stage[q * 64 + tid]);
+      sm.O[(tid >> 3) * S::LDO + (tid & 7)] = v;
+    }
+  } else {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int i = ui + 4 * r;
-      if (i < N && i != N - 1) sO[i][uj] = cmul(sO[i][uj], m);
-    }
-  }
-  __syncthreads();
-  // ---- log|det| and phase from the pivots, one per lane of warp 0
-  if (tid < 32) {
-    double la = 0.0;
-    double2 ph = make_double2(1.0, 0.0);
-    if (tid < N) {
-      const double2 u = sPiv[tid];
-      const double a = cabs_(u);
-      la = log(a);
-      ph = make_double2(u.x / a, u.y / a);
-    }
+    for (int j = 0; j < CT; ++j)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      la += __shfl_xor_sync(0xffffffffu, la, o);
-      const double2 q = make_double2(__shfl_xor_sync(0xffffffffu, ph.x, o), __shfl_xor_sync(0xffffffffu, ph.y, o));
-      ph = cmul(ph, q);
-    }
-    if (tid == 0) {
-      red[0] = make_double2(la, 0.0);
-      red[1] = (swaps & 1) ? make_double2(-ph.x, -ph.y) : ph;
-    }
+      for (int q = 0; q < 2; ++q)
+        sm.O[(rt * 8 + g) * S::LDO + (ct0 + j) * 8 + 2 * t + q] = make_double2(re[j][q], im[j][q]);
   }
-  __syncthreads();
-  SpinDet32 out;
-  out.logabs = red[0].x;
-  out.phase = red[1];
-  return out;
 }
 
-// Ghalf (N, M) of one spin block from X = (P O)^-1 in sO: Ghalf[i, m] = sum_r X[i, r] phi[m, perm(r)].
-// The steps (pass of 64 columns m, group of kRC permuted columns) run in one sequence through
-// the copy ring, passes included.
-__device__ void ghalf_block(const double2* __restrict__ phi, int M, int N, double2 (*sO)[kNP], const int* sPerm,
-                            double2* sStage, double2* __restrict__ ghalf, double2* __restrict__ ghalf2) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int i0 = warp * 8;  // this warp's rows
-  // the next step to copy: columns from im0, permuted columns from ir0 (im0 >= M: none left)
-  int im0 = 0, ir0 = 0, slot = 0;
-  // phi[im0 + ml][perm(ir0 + rr)] as sPT[rr][ml] (consecutive threads take consecutive rr)
-  auto issue = [&]() {
-    if (im0 < M) {
-      double2* sPT = sStage + slot * kGStage;
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// Gauss-Jordan inverse of the N x N block in sm.O (see above); sm.perm, sm.inv, sm.piv.
+template <int NT>
+__device__ __forceinline__ void gf_invert(int N, GfShared<NT>& sm, unsigned* status) {
+  using S = GfShape<NT>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  if (tid < 32) {
+    sm.perm[tid] = sm.inv[tid] = tid;
+    if (tid == 0) sm.used = 0u;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int kb = 0; kb < NT; ++kb) {
+    if (warp == kb % S::WARPS) {
+      double2 a[8];
+      const int row = lane < S::NP ? lane : 0;
 #pragma unroll
-      for (int u = 0; u < kRC * 32 * kMQ / kThreads; ++u) {
-        const int e = tid + u * kThreads, rr = e % kRC, ml = e / kRC;
-        const int r = ir0 + rr, m = im0 + ml;
-        const bool in = r < N && m < M;
-        cp_async16(sPT + rr * kMS + ml, phi + (in ? (size_t)m * N + sPerm[r] : 0), in ? 16 : 0);
-      }
-      ir0 += kRC;
-      if (ir0 >= N) {
-        ir0 = 0;
-        im0 += 32 * kMQ;
-      }
-    }
-    cp_async_commit();
-    slot = slot == kGRing - 1 ? 0 : slot + 1;
-  };
-  issue();
-  issue();
-  issue();
-  int cur = 0;  // ring slot of the step being multiplied
-  for (int m0 = 0; m0 < M; m0 += 32 * kMQ) {
-    double2 acc[8][kMQ];
+      for (int j = 0; j < 8; ++j) a[j] = sm.O[row * S::LDO + 8 * kb + j];
+      unsigned used = sm.used;
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+      for (int jj = 0; jj < 8; ++jj) {
+        const int k = 8 * kb + jj;
+        if (k < N) {
+          unsigned key = 0u;
+          const double2 own = a[jj];
+          if (lane < N && !((used >> lane) & 1u))
+            key = (__float_as_uint((float)cabs2(own)) & ~31u) | (unsigned)(31 - lane);
+          // every lane scales its row as if it held the pivot, while the pivot is found
+          const double rn = __drcp_rn(own.x * own.x + own.y * own.y);
+          const double2 pinv = make_double2(own.x * rn, -own.y * rn);
+          double2 s[8];
 #pragma unroll
-      for (int q = 0; q < kMQ; ++q) acc[a][q] = make_double2(0.0, 0.0);
-    for (int r0 = 0; r0 < N; r0 += kRC) {
-      cp_async_wait<2>();
-      __syncthreads();
-      issue();  // into the slot of the previous step
-      const double2* sPT = sStage + cur * kGStage;
-      cur = cur == kGRing - 1 ? 0 : cur + 1;
+          for (int j = 0; j < 8; ++j) s[j] = j == jj ? pinv : cmul(a[j], pinv);
+          key = __reduce_max_sync(0xffffffffu, key);
+          int p = 31 - (int)(key & 31u);
+          if (key < 32u) {
+            // no positive |a|^2 left (an exactly singular block, or NaN): any free row
+            p = __ffs(~used) - 1;
+          }
+          const bool mine = lane == p;
+          if (mine) {
+            if (own.x == 0.0 && own.y == 0.0) flag(status, STATUS_SINGULAR);
+            sm.piv[k] = own;
+            sm.perm[k] = lane;
+            sm.inv[lane] = k;
+          }
+          used |= 1u << p;
 #pragma unroll
-      for (int rr = 0; rr < kRC; ++rr) {
-        double2 x[8];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) x[a] = sO[i0 + a][min(r0 + rr, 31)];
-        if (r0 + rr >= N) continue;  // uniform
-#pragma unroll
-        for (int q = 0; q < kMQ; ++q) {
-          if (q > 0 && m0 + 32 * q >= M) break;  // a column group wholly past M (uniform): the last pass
-          const double2 b = sPT[rr * kMS + lane + 32 * q];
-#pragma unroll
-          for (int a = 0; a < 8; ++a) {
-            acc[a][q].x += x[a].x * b.x - x[a].y * b.y;
-            acc[a][q].y += x[a].x * b.y + x[a].y * b.x;
+          for (int j = 0; j < 8; ++j) {
+            const double2 r = shfl2(s[j], p);
+            if (mine) {
+              a[j] = s[j];
+            } else if (j == jj) {
+              const double2 v = cmul(own, r);
+              a[j] = make_double2(-v.x, -v.y);
+            } else {
+              a[j] = csub(a[j], cmul(own, r));
+            }
           }
         }
       }
+      if (lane < S::NP) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          sm.P[lane * S::LDP + j] = a[j];
+          sm.O[lane * S::LDO + 8 * kb + j] = a[j];
+        }
+      }
+      if (lane == 0) sm.used = used;
     }
+    if (NT == 1) break;
+    __syncthreads();
+    // rank-8 update of the other columns.  Row tile rt, column tiles ct0, ct0 + 1, ... but kb
+    constexpr int CT = NT >= 3 ? NT : 1;
+    const int rt = NT >= 3 ? warp : (warp & 1), ct0 = NT == 2 ? (warp >> 1) : 0;
+    double2 b[CT][2];  // pivot rows of the columns, before anyone rewrites them
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int i = i0 + a;
-      if (i >= N) break;
+    for (int j = 0; j < CT; ++j)
 #pragma unroll
-      for (int q = 0; q < kMQ; ++q) {
-        const int m = m0 + lane + 32 * q;
-        if (m < M) {
-          ghalf[(size_t)i * M + m] = acc[a][q];
-          if (ghalf2 != nullptr) ghalf2[(size_t)i * M + m] = acc[a][q];
+      for (int h = 0; h < 2; ++h) b[j][h] = sm.O[sm.perm[8 * kb + 4 * h + t] * S::LDO + 8 * (ct0 + j) + g];
+    const int row = rt * 8 + g;
+    bool pivot = false;
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) pivot |= sm.perm[8 * kb + jj] == row;
+    const double2 a0 = sm.P[row * S::LDP + t], a1 = sm.P[row * S::LDP + 4 + t];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+      if (ct0 + j == kb) continue;
+      double2* c = sm.O + row * S::LDO + 8 * (ct0 + j) + 2 * t;
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+      if (!pivot) {
+        const double2 c0 = c[0], c1 = c[1];
+        re[0] = c0.x;
+        re[1] = c1.x;
+        im[0] = c0.y;
+        im[1] = c1.y;
+      }
+      dmma884(re, a0.x, b[j][0].x);
+      dmma884(im, a0.x, b[j][0].y);
+      dmma884(re, -a0.y, b[j][0].y);
+      dmma884(im, a0.y, b[j][0].x);
+      dmma884(re, a1.x, b[j][1].x);
+      dmma884(im, a1.x, b[j][1].y);
+      dmma884(re, -a1.y, b[j][1].y);
+      dmma884(im, a1.y, b[j][1].x);
+      c[0] = make_double2(re[0], im[0]);
+      c[1] = make_double2(re[1], im[1]);
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+}
+
+// log|det O| and its phase from the pivots and the parity of the pivot order, by warp 0:
+// sm.red[0].x, sm.red[1].
+template <int NT>
+__device__ __forceinline__ void gf_determinant(int N, GfShared<NT>& sm) {
+  const int lane = threadIdx.x;
+  if (lane >= 32) return;
+  double la = 0.0;
+  double2 ph = make_double2(1.0, 0.0);
+  const int p = sm.perm[lane];
+  int inversions = 0;
+#pragma unroll 8
+  for (int j = 1; j < 8 * NT; ++j) inversions += (j > lane && sm.perm[j] < p) ? 1 : 0;
+  if (lane < N) {
+    const double2 u = sm.piv[lane];
+    const double a = cabs_(u);
+    la = log(a);
+    ph = make_double2(u.x / a, u.y / a);
+    if (inversions & 1) ph = make_double2(-ph.x, -ph.y);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    la += __shfl_xor_sync(0xffffffffu, la, o);
+    ph = cmul(ph, make_double2(__shfl_xor_sync(0xffffffffu, ph.x, o), __shfl_xor_sync(0xffffffffu, ph.y, o)));
+  }
+  if (lane == 0) {
+    sm.red[0] = make_double2(la, 0.0);
+    sm.red[1] = ph;
+  }
+}
+
+template <int NT>
+__device__ __forceinline__ void gf_ghalf(const double2* __restrict__ phi, int M, int N, GfShared<NT>& sm,
+                                         double2* __restrict__ ghalf, double2* __restrict__ ghalf2) {
+  using S = GfShape<NT>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nch = (M + S::GM - 1) / S::GM;
+  auto issue = [&](int ch) {
+    if (ch < nch) {
+      double2* st = sm.stage + (ch % S::RING) * S::GSTAGE;
+      for (int e = tid; e < S::GM * S::NP; e += S::THREADS) {
+        const int r = e / S::NP, c = e % S::NP, m = ch * S::GM + r;
+        const bool in = m < M && c < N;
+        cp_async16(st + r * S::LDG + c, phi + (in ? (size_t)m * N + c : 0), in ? 16 : 0);
+      }
+    }
+    cp_async_commit();
+  };
+  issue(0);
+  issue(1);
+  const int rt = warp % NT, mw = warp / NT, i = rt * 8 + g;
+  double2 a[2 * NT];
+#pragma unroll
+  for (int k = 0; k < 2 * NT; ++k) a[k] = sm.O[sm.perm[i] * S::LDO + sm.inv[4 * k + t]];
+  const int col = 4 * (g & 1) + (g >> 1);  // row of phi behind MMA column g
+  for (int ch = 0; ch < nch; ++ch) {
+    cp_async_wait<1>();
+    __syncthreads();
+    issue(ch + 2);
+#pragma unroll
+    for (int mt = 0; mt < S::GM / 8; ++mt) {
+      if (S::MW > 1 && mt % S::MW != mw) continue;
+      const int m0 = ch * S::GM + 8 * mt;
+      if (m0 >= M) break;
+      const double2* b = sm.stage + (ch % S::RING) * S::GSTAGE + (8 * mt + col) * S::LDG + t;
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 2 * NT; ++k) {
+        const double2 bv = b[4 * k];
+        dmma884(re, a[k].x, bv.x);
+        dmma884(im, a[k].x, bv.y);
+        dmma884(re2, -a[k].y, bv.y);
+        dmma884(im2, a[k].y, bv.x);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int m = m0 + 4 * q + t;
+        if (i < N && m < M) {
+          const double2 v = make_double2(re[q] + re2[q], im[q] + im2[q]);
+          ghalf[(size_t)i * M + m] = v;
+          if (ghalf2 != nullptr) ghalf2[(size_t)i * M + m] = v;
         }
       }
     }
@@ -312,48 +410,42 @@ __device__ void ghalf_block(const double2* __restrict__ phi, int M, int N, doubl
   cp_async_wait<0>();
 }
 
-template <bool WITH_GHALF>
-__global__ void __launch_bounds__(kThreads, 4) gf_lu32_kernel(const double2* __restrict__ phia,
-                                                              const double2* __restrict__ phib, int M, int na,
-                                                              int nb, const double2* __restrict__ psia_c,
-                                                              const double2* __restrict__ psib_c,
-                                                              const double* __restrict__ log_shift,
-                                                              double2* __restrict__ ghalfa,
-                                                              double2* __restrict__ ghalfb,
-                                                              double2* __restrict__ ovlp, double2* __restrict__ logdet,
-                                                              unsigned* status) {
-  __shared__ double2 sO[32][kNP];
-  __shared__ __align__(16) double2 sStage[kStage];  // the O product's chunk ring, then the Ghalf step ring
-  __shared__ double2 sPiv[32];
-  __shared__ double2 red[8];
-  __shared__ int sPerm[32];
+template <int NT, bool WITH_GHALF>
+__global__ void __launch_bounds__(GfShape<NT>::THREADS, 4)
+    gf_mma_kernel(const double2* __restrict__ phia, const double2* __restrict__ phib, int M, int na, int nb,
+                  const double2* __restrict__ psia_c, const double2* __restrict__ psib_c,
+                  const double* __restrict__ log_shift, double2* __restrict__ ghalfa, double2* __restrict__ ghalfb,
+                  double2* __restrict__ ovlp, double2* __restrict__ logdet, unsigned* status) {
+  extern __shared__ __align__(16) unsigned char gf_sm[];
+  GfShared<NT>& sm = *reinterpret_cast<GfShared<NT>*>(gf_sm);
   const int w = blockIdx.x;
   // spin aliasing: phib == phia with nb == na is one block counted twice
   const bool alias = (phib == phia) && (nb == na);
   double logsum = 0.0;
-  double2 phase = make_double2(1.0, 0.0);
+  double2 phase = make_double2(1.0, 0.0);  // (thread 0's are used)
   for (int s = 0; s < 2; ++s) {
     const int N = s == 0 ? na : nb;
     if (N == 0) continue;
     if (s == 1 && alias) {
-      logsum += red[2].x;
-      phase = cmul(phase, red[3]);
+      logsum += logsum;
+      phase = cmul(phase, phase);
       if (logdet != nullptr && threadIdx.x == 0) logdet[(size_t)w * 2 + 1] = logdet[(size_t)w * 2];
       continue;
     }
     const double2* phi = (s == 0 ? phia : phib) + (size_t)w * M * N;
-    const SpinDet32 d = invert_block(phi, s == 0 ? psia_c : psib_c, M, N, sO, sStage, sPerm, sPiv, red, status);
-    logsum += d.logabs;
-    phase = cmul(phase, d.phase);
+    gf_overlap_tiles<NT>(phi, s == 0 ? psia_c : psib_c, M, N, sm);
+    __syncthreads();
+    gf_invert<NT>(N, sm, status);
+    gf_determinant<NT>(N, sm);
     if (threadIdx.x == 0) {
-      red[2] = make_double2(d.logabs, 0.0);
-      red[3] = d.phase;
-      if (logdet != nullptr) logdet[(size_t)w * 2 + s] = make_double2(d.logabs, atan2(d.phase.y, d.phase.x));
+      logsum += sm.red[0].x;
+      phase = cmul(phase, sm.red[1]);
+      if (logdet != nullptr) logdet[(size_t)w * 2 + s] = make_double2(sm.red[0].x, atan2(sm.red[1].y, sm.red[1].x));
     }
     if (WITH_GHALF) {
       double2* g1 = (s == 0 ? ghalfa : ghalfb) + (size_t)w * N * M;
       double2* g2 = (s == 0 && alias && nb > 0 && ghalfb != ghalfa) ? ghalfb + (size_t)w * N * M : nullptr;
-      ghalf_block(phi, M, N, sO, sPerm, sStage, g1, g2);
+      gf_ghalf<NT>(phi, M, N, sm, g1, g2);
     }
     __syncthreads();
   }
@@ -362,6 +454,20 @@ __global__ void __launch_bounds__(kThreads, 4) gf_lu32_kernel(const double2* __r
     if (!finite2(o)) flag(status, STATUS_NONFINITE);
     ovlp[w] = o;
   }
+}
+
+template <int NT>
+cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M, int na, int nb,
+                          const double2* psia_c, const double2* psib_c, const double* log_shift, double2* ghalfa,
+                          double2* ghalfb, double2* ovlp, double2* logdet, unsigned* status, cudaStream_t st) {
+  const int smem = (int)sizeof(GfShared<NT>);
+  auto k = ghalfa != nullptr ? gf_mma_kernel<NT, true> : gf_mma_kernel<NT, false>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k<<<W, GfShape<NT>::THREADS, smem, st>>>(phia, phib, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp,
+                                           logdet, status);
+  note_launch();
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -545,14 +651,12 @@ cudaError_t launch_gf_lu32(const double2* phia, const double2* phib, int W, int 
                            const double2* psia_c, const double2* psib_c, const double* log_shift, double2* ghalfa,
                            double2* ghalfb, double2* ovlp, double2* logdet, unsigned* status, cudaStream_t st) {
   if (!gf_lu32_fits(na, nb) || M <= 0 || W <= 0) return cudaErrorInvalidValue;
-  if (ghalfa != nullptr)
-    gf_lu32_kernel<true><<<W, kThreads, 0, st>>>(phia, phib, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb,
-                                                 ovlp, logdet, status);
-  else
-    gf_lu32_kernel<false><<<W, kThreads, 0, st>>>(phia, phib, M, na, nb, psia_c, psib_c, log_shift, nullptr,
-                                                  nullptr, ovlp, logdet, status);
-  note_launch();
-  return cudaGetLastError();
+  switch ((max(na, nb) + 7) / 8) {
+    case 1: return launch_gf_mma<1>(phia, phib, W, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp, logdet, status, st);
+    case 2: return launch_gf_mma<2>(phia, phib, W, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp, logdet, status, st);
+    case 3: return launch_gf_mma<3>(phia, phib, W, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp, logdet, status, st);
+    default: return launch_gf_mma<4>(phia, phib, W, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp, logdet, status, st);
+  }
 }
 
 cudaError_t launch_reortho_chol32(double2* phia, double2* phib, int W, int M, int na, int nb,

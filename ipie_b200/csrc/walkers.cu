@@ -278,7 +278,7 @@ __device__ __forceinline__ double2 shift_one(double2 v, double2 m, double r, dou
 // that both sides move whole 128-byte lines.  The share is one of a cluster's S (the host's choice:
 // about four CTAs per SM, 64 fields or more each), whose partial sums are added through distributed
 // shared memory in rank order.  The first version, one CTA per 32 walkers over all of X, ran 2 to 32
-// CTAs: 84 -> 9 us at 640 walkers, X = 600; 37 -> 5.4 us at 256 walkers, X = 320; 14.7 -> 3.6 us at 64
+// CTAs: 84 -> 13.5 us at 640 walkers, X = 600; 37 -> 5.4 us at 256 walkers, X = 320; 14.7 -> 3.6 us at 64
 // walkers, X = 120.
 constexpr int kShiftWalkers = 8, kShiftStep = 64;
 __global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restrict__ vbias,
