@@ -524,11 +524,13 @@ __device__ __forceinline__ uint32_t split2_f16(float y0, float y1, uint32_t& lo)
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// The epilogue goes through shared memory and TMA tensor stores: one 32 KB staging box of 64
+// The epilogue goes through shared memory and TMA tensor stores: two 32 KB staging boxes of 64
 // walkers x 16 rows x 16 halves (the {16, 16, 64} box of the plane maps maps->out: re_hi, re_lo,
-// im_hi, im_lo), filled and stored eight times per tile -- real then imaginary plane, the
-// transposed block (J, I) then the block (I, J), head then remainder -- by the threads of the
-// rows (c) that feed that plane.  A thread's scattered 16-byte global stores (one 32-byte sector
+// im_hi, im_lo), one for the real plane (filled by the rows c = 1) and one for the imaginary (c = 0),
+// filled and stored four times per tile -- the transposed block (J, I) then the block (I, J), head
+// then remainder.  (One box, eight times, kept half the threads idle: 24.7 -> 21.1 us at 512 walkers,
+// M = 76, 116 -> 104 us at 700 walkers, M = 132; equal at 2048 walkers, M = 200, 1.14 ms.)  A thread's
+// scattered 16-byte global stores (one 32-byte sector
 // split between two of them, 16 walkers per warp instruction) took ~30k cycles per tile and
 // stalled the next tile's products; the staged tensor stores leave the copy to the TMA engine.
 // Rows i >= M and columns j >= ld of a box are clipped by the store.
@@ -536,14 +538,14 @@ __device__ __forceinline__ uint32_t split2_f16(float y0, float y1, uint32_t& lo)
 // Bank spread: a walker's part of the box is 512 bytes, so the 16 walkers of a warp instruction
 // would all write the same four banks if each wrote the same 16-byte chunk of its part.  Lane k
 // (k = (lane / 2) mod 8) writes its chunks in an order rotated by k instead: its block chunks
-// (8 rows x two 16-byte halves) rotated by k within each half of eight, which spreads the 16
-// lanes over all 32 banks (two wavefronts per instruction), and the transposed rows b rotated by
-// k mod 4 within each group of four (four wavefronts: a transposed row has one 16-byte half per
-// column group).  The values are split into head and remainder once per tile.
+// (8 rows x two 16-byte halves) rotated by k within each half of eight, which spreads the lanes
+// over all 32 banks (four wavefronts per instruction of 512 bytes), and the transposed rows b rotated by
+// k mod 4 within each group of four (a transposed row has one 16-byte half per column group).  The values are split into head and remainder once per tile.
 struct EpiVHSBlock {
   int M, W, nb;  // nb: 16-orbital blocks per side
   float f;       // sqrt(dt) v_scale / (operand scales)
-  static constexpr int kSmemBytes = 64 * 16 * 32;
+  static constexpr int kBox = 64 * 16 * 32;
+  static constexpr int kSmemBytes = 2 * kBox;
   static constexpr bool kUsesMaps = true;
   static constexpr int kThreads = 256;  // the epilogue threads of the 128 x 256 tile (barrier 3)
   __device__ __forceinline__ static void sync() { asm volatile("bar.sync 3, %0;\n" ::"r"(kThreads) : "memory"); }
@@ -605,37 +607,35 @@ struct EpiVHSBlock {
     const int g = (col0 >> 7) & 1;
     const float s = c ? -f : f;
     const int k = (threadIdx.x >> 1) & 7;
-    uint8_t* mine = smem + wl * 512;
+    // the rows c = 1 feed the real plane, c = 0 the imaginary one: one box each per round
+    uint8_t* mine = smem + (1 - c) * kBox + wl * 512;
     // head / remainder pairs: word 8 a + m holds columns 2m, 2m + 1 of the thread's row a
     uint32_t ph[64], pl[64];
 #pragma unroll
     for (int e = 0; e < 64; ++e) ph[e] = split2_f16(v[2 * e] * s, v[2 * e + 1] * s, pl[e]);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int pc = 1 - half;  // the rows feeding this plane: c = 1 real, c = 0 imaginary
-      const bool act = live && c == pc;
+    for (int rd = 0; rd < 4; ++rd) {
+      const int tr = rd < 2, lo = rd & 1;
+      if (tr && I == J) continue;  // the same for every thread of the tile
+      if (rd == 2) {
+        rotate(ph, k);
+        rotate(pl, k);
+      }
+      if (threadIdx.x == 0) bulk_wait_read_all();  // the previous boxes have left shared memory
+      sync();
+      if (live) {
+        if (lo)
+          put(pl, tr, k, g, mine);
+        else
+          put(ph, tr, k, g, mine);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      }
+      sync();
+      if (threadIdx.x == 0) {
 #pragma unroll
-      for (int rd = 0; rd < 4; ++rd) {
-        const int tr = rd < 2, lo = rd & 1;
-        if (tr && I == J) continue;  // the same for every thread of the tile
-        if (rd == 2 && act) {
-          rotate(ph, k);
-          rotate(pl, k);
-        }
-        if (threadIdx.x == 0) bulk_wait_read_all();  // the previous box has left shared memory
-        sync();
-        if (act) {
-          if (lo)
-            put(pl, tr, k, g, mine);
-          else
-            put(ph, tr, k, g, mine);
-          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        }
-        sync();
-        if (threadIdx.x == 0) {
-          tma_store_3d(&maps->out[(pc ? 0 : 2) + lo], tr ? 16 * I : 16 * J, tr ? 16 * J : 16 * I, w0, smem);
-          bulk_commit();
-        }
+        for (int pc = 0; pc < 2; ++pc)
+          tma_store_3d(&maps->out[2 * pc + lo], tr ? 16 * I : 16 * J, tr ? 16 * J : 16 * I, w0, smem + pc * kBox);
+        bulk_commit();
       }
     }
   }
@@ -1118,8 +1118,9 @@ cudaError_t mixed_vhs_blocks(const void* cb_hi, const void* cb_lo, int X, int M,
   for (int p = 0; p < 4; ++p)
     if ((e = make_map_f16_store(&maps.out[p], planes[p], W, M, f16_ld(M), 16, 16, 64)) != cudaSuccess) return e;
   const EpiVHSBlock epi{M, W, (M + 15) / 16, (float)(sqrt_dt / (cb_scale * kFieldScaleF16) * v_scale)};
-  // 64-byte K rows: four 48 KB stages instead of two of 96 KB, so that three are in flight
-  return launch_umma<BN, 1, 3, 4, EpiVHSBlock, KIND_F16_K32>(maps, X, 0, 0, grid, epi, status, st, true,
+  // 64-byte K rows: three 48 KB stages (four, and two of 96 KB, ran the main loop no faster) leave
+  // room for two boxes in the epilogue
+  return launch_umma<BN, 1, 3, 3, EpiVHSBlock, KIND_F16_K32>(maps, X, 0, 0, grid, epi, status, st, true,
                                                             persistent != 0);
 }
 
