@@ -1,5 +1,5 @@
 // Green's function, overlap and reorthogonalisation for spin blocks of N <= 32 electrons: one CTA of
-// 96 or 128 threads per walker, four per SM, the products on the f64 tensor cores.
+// 96 or 128 threads per walker, four per SM, on the f64 tensor cores.
 // ovlp_w = prod_s phase_s * exp(sum_s log|det O_s| - log_shift_w).
 // Same contracts as gf_overlap_kernel and reortho_kernel (walkers.cu), which keep N > 32.
 #include "common.cuh"
@@ -9,86 +9,7 @@ namespace ipie_b200 {
 
 namespace {
 
-constexpr int kThreads = 128;
-constexpr int kChunk = 8;   // rows of phi / psi* per shared-memory chunk of the O product
-constexpr int kORing = 3;   // chunks in the O product's copy ring
-constexpr int kNP = 33;     // row stride of O in shared memory
-constexpr int kRC = 4;      // permuted columns of phi per staged step of the Ghalf product
-constexpr int kMQ = 2;      // columns of Ghalf per lane and pass (64 per pass)
-constexpr int kMS = 32 * kMQ + 1;  // row stride of the staged phi^T step (odd in 16-byte units)
-constexpr int kGRing = 4;   // steps in the Ghalf product's copy ring
-constexpr int kOStage = 2 * kChunk * 32;  // double2 per O chunk (phi and psi*)
-constexpr int kGStage = kRC * kMS;        // double2 per Ghalf step
-constexpr int kStage = kORing * kOStage > kGRing * kGStage ? kORing * kOStage : kGRing * kGStage;
-static_assert(kChunk * 32 % kThreads == 0 && kRC * 32 * kMQ % kThreads == 0, "whole copies per thread");
-
-struct SpinDet32 {
-  double logabs;
-  double2 phase;
-};
-
-// sO = phi^T psi* (or, GRAM, the Gram matrix phi^H phi: psic unused) of one spin block.  phi and
-// psi* stream through shared memory in 8-row chunks, a three-deep ring of cp.async copies issued
-// two chunks ahead (one barrier per chunk); thread (ti, tj) accumulates rows {ti, ti+16} x
-// columns {tj + 8q} in registers.  The caller synchronises before reading sO.
-template <bool GRAM>
-__device__ void o_product(const double2* __restrict__ phi, const double2* __restrict__ psic, int M, int N,
-                          double2 (*sO)[kNP], double2* sStage) {
-  const int tid = threadIdx.x;
-  const int ti = tid >> 3, tj = tid & 7;
-  double2 acc[2][4];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[a][q] = make_double2(0.0, 0.0);
-  const int nch = (M + kChunk - 1) / kChunk;
-  // chunk ch (rows 8 ch ..) into ring slot ch % kORing: phi rows then psi* rows, zeros past M / N
-  auto issue = [&](int ch) {
-    if (ch < nch) {
-      double2* st = sStage + (ch % kORing) * kOStage;
-#pragma unroll
-      for (int u = 0; u < kChunk * 32 / kThreads; ++u) {
-        const int e = tid + u * kThreads, r = e >> 5, c = e & 31, m = ch * kChunk + r;
-        const bool in = m < M && c < N;
-        const size_t off = in ? (size_t)m * N + c : 0;
-        cp_async16(st + e, phi + off, in ? 16 : 0);
-        if (!GRAM) cp_async16(st + kChunk * 32 + e, psic + off, in ? 16 : 0);
-      }
-    }
-    cp_async_commit();  // (an empty group past the end keeps the group count per chunk)
-  };
-  issue(0);
-  issue(1);
-  for (int ch = 0; ch < nch; ++ch) {
-    cp_async_wait<1>();  // this thread's copies of chunk ch have landed
-    __syncthreads();     // everyone's have, and everyone is done with chunk ch - 1
-    issue(ch + 2);       // into the slot of chunk ch - 1
-    const double2(*sPhi)[32] = reinterpret_cast<const double2(*)[32]>(sStage + (ch % kORing) * kOStage);
-    const double2(*sPsi)[32] =
-        GRAM ? sPhi : reinterpret_cast<const double2(*)[32]>(sStage + (ch % kORing) * kOStage + kChunk * 32);
-#pragma unroll
-    for (int r = 0; r < kChunk; ++r) {
-      double2 a0 = sPhi[r][ti], a1 = sPhi[r][ti + 16];
-      if (GRAM) {
-        a0.y = -a0.y;
-        a1.y = -a1.y;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double2 b = sPsi[r][tj + 8 * q];
-        acc[0][q].x += a0.x * b.x - a0.y * b.y;
-        acc[0][q].y += a0.x * b.y + a0.y * b.x;
-        acc[1][q].x += a1.x * b.x - a1.y * b.y;
-        acc[1][q].y += a1.x * b.y + a1.y * b.x;
-      }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sO[ti + 16 * a][tj + 8 * q] = acc[a][q];
-}
+constexpr int kChunk = 8;  // rows of phi / psi* per shared-memory chunk of the overlap and Gram products
 
 // ---------------------------------------------------------------------------------------------
 // The Green's function on the f64 tensor cores, N padded to NT tiles of 8.  Per walker and spin:
@@ -472,133 +393,288 @@ cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M
 
 // ---------------------------------------------------------------------------------------------
 // Reorthogonalisation of spin blocks of N <= 32 orbitals by Cholesky QR, the same unique thin QR
-// (positive real diag R) as Gram-Schmidt or a sign-fixed Householder factorisation:
-//   S = phi^H phi (o_product<true>), S = R^H R (Cholesky, right-looking, in shared memory; warp 0
-//   scales the pivot row, all threads update the trailing upper triangle), X = R^-1 (warp 0,
-//   lane i solving row i of X R = I, kept in the lower triangle of sO transposed plus the
-//   diagonal), phi <- phi X in place (16-row chunks of phi through the copy ring; lane i forms
-//   column i of four rows per warp, so each output row is one coalesced 512-byte store).
-// log det R = sum log R_kk.  Its error is that of the Gram matrix, ~cond(phi)^2 eps: walkers are
+// (positive real diag R) as Gram-Schmidt or a sign-fixed Householder factorisation, on the f64
+// tensor cores (N padded to NT tiles of 8):
+//   S = phi^H phi (lower tiles): chunks of 8 rows of phi through a cp.async ring;
+//   S = L L^H (L = R^H) and W = L^-1 in panels of 8 columns: one warp factors the panel with a row
+//       per lane (shuffles, no barriers) and inverts its diagonal block D = L_KK^-1, then all warps
+//       apply it as 8 x 8 x 8 products, three barriers per panel:
+//         W[K, J] <- D W[K, J] (J < K),  S[I, J] -= L[I, K] L[J, K]^H (I >= J > K),
+//         W[I, J] -= L[I, K] W[K, J] (I > K, J <= K).
+//       W replaces S tile by tile in sm.O (column block J of S is spent once panel J is factored);
+//   phi <- phi W^H in place, chunks of 32 rows, a row tile per warp, the zero tiles of W skipped.
+// log det R = sum log L_kk.  Its error is that of the Gram matrix, ~cond(phi)^2 eps: walkers are
 // reorthogonalised every few steps, so phi stays close to orthonormal and cond(phi) near 1.
-__device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, int N, double2 (*sO)[kNP], double2* sStage,
-                               double2* sDinv, double* sSpread, unsigned* status) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  o_product<true>(phi, nullptr, M, N, sO, sStage);
+// 2048 walkers, M = 200, N = 32: 537 -> 291 us (419 MB of orbitals in and out: 63 us; the products' floor is
+// 100 us); 512, M = 76, N = 10: 72 -> 20 us (against DFMA products, a barrier pair per Cholesky column and
+// a serial triangular inverse).
+template <int NT>
+struct RoShape {
+  static constexpr int WARPS = NT == 3 ? 3 : 4, THREADS = 32 * WARPS, NP = 8 * NT;
+  static constexpr int LDO = NP + 4, LDP = 12;
+  static constexpr int LDC = NP + 2;      // chunks of the Gram product (2 mod 8)
+  static constexpr int LDX = NP + 4;      // chunks of phi W^H (4 mod 8)
+  static constexpr int XM = 8 * WARPS;    // rows of phi per chunk of phi W^H
+  static constexpr int RING = 3;
+  static constexpr int CSTAGE = kChunk * LDC, XSTAGE = XM * LDX;
+  static constexpr int XRING = NT == 4 ? 2 : 3;  // (two keep four walkers of 32 electrons on an SM)
+  static constexpr int STAGE = RING * CSTAGE > XRING * XSTAGE ? RING * CSTAGE : XRING * XSTAGE;
+  static_assert(STAGE >= (NP + 8) * LDP, "the panel and its diagonal inverse live in the rings' room");
+  static constexpr int UNITS = NT * (NT + 1) / 2, PER = (UNITS + WARPS - 1) / WARPS;  // lower tiles, per warp
+};
+
+template <int NT>
+struct RoShared {
+  using S = RoShape<NT>;
+  double2 O[S::NP * S::LDO];
+  union {
+    double2 stage[S::STAGE];  // copy rings of the two products with phi
+    struct {                  // between them
+      double2 P[S::NP * S::LDP];
+      double2 D[8 * S::LDP];
+    };
+  };
+  double diag[32];
+  double spread, logsum;
+};
+
+// row and column tile of lower tile u (row-major over J <= I)
+__device__ __forceinline__ void lower_tile(int u, int& I, int& J) {
+  I = u < 1 ? 0 : u < 3 ? 1 : u < 6 ? 2 : 3;
+  J = u - I * (I + 1) / 2;
+}
+
+// (re, im) of one 8 x 8 tile += a b over 4 columns of k
+__device__ __forceinline__ void cmma(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+  dmma884(re, a.x, b.x);
+  dmma884(im, a.x, b.y);
+  dmma884(re, -a.y, b.y);
+  dmma884(im, a.y, b.x);
+}
+__device__ __forceinline__ double2 conj_(double2 z) { return make_double2(z.x, -z.y); }
+
+template <int NT>
+__device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, int N, RoShared<NT>& sm,
+                                            unsigned* status) {
+  using S = RoShape<NT>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  // ---- S = phi^H phi, tile (I, J) = sum_m conj(phi[m, I]) phi[m, J]
+  {
+    const int nch = (M + kChunk - 1) / kChunk;
+    auto issue = [&](int ch) {
+      if (ch < nch) {
+        double2* st = sm.stage + (ch % S::RING) * S::CSTAGE;
+        for (int e = tid; e < kChunk * S::NP; e += S::THREADS) {
+          const int r = e / S::NP, c = e % S::NP, m = ch * kChunk + r;
+          const bool in = m < M && c < N;
+          cp_async16(st + r * S::LDC + c, phi + (in ? (size_t)m * N + c : 0), in ? 16 : 0);
+        }
+      }
+      cp_async_commit();
+    };
+    double re[S::PER][2], im[S::PER][2];
+    int arow[S::PER], bcol[S::PER];
+#pragma unroll
+    for (int q = 0; q < S::PER; ++q) {
+      re[q][0] = re[q][1] = im[q][0] = im[q][1] = 0.0;
+      int I, J;
+      lower_tile(min(warp + q * S::WARPS, S::UNITS - 1), I, J);
+      arow[q] = t * S::LDC + 8 * I + g;
+      bcol[q] = t * S::LDC + 8 * J + g;
+    }
+    issue(0);
+    issue(1);
+    for (int ch = 0; ch < nch; ++ch) {
+      cp_async_wait<1>();
+      __syncthreads();
+      issue(ch + 2);
+      const double2* st = sm.stage + (ch % S::RING) * S::CSTAGE;
+#pragma unroll
+      for (int kk = 0; kk < kChunk; kk += 4)
+#pragma unroll
+        for (int q = 0; q < S::PER; ++q) {
+          if (warp + q * S::WARPS >= S::UNITS) break;
+          cmma(re[q], im[q], conj_(st[arow[q] + kk * S::LDC]), st[bcol[q] + kk * S::LDC]);
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int q = 0; q < S::PER; ++q) {
+      if (warp + q * S::WARPS >= S::UNITS) break;
+      int I, J;
+      lower_tile(warp + q * S::WARPS, I, J);
+      // S[j, i] = conj(S[i, j]): with rows I and columns J of phi^H phi this is the lower tile
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        sm.O[(8 * I + g) * S::LDO + 8 * J + 2 * t + h] = make_double2(re[q][h], im[q][h]);
+    }
+  }
   __syncthreads();
-  // ---- S = R^H R in the upper triangle of sO
-  const int uj = tid & 31, ui = tid >> 5;
-  for (int k = 0; k < N; ++k) {
-    if (tid < 32) {
-      const double skk = sO[k][k].x;
-      __syncwarp();  // every lane has read the pivot before lane 0 replaces it
-      if (!(skk > 0.0)) flag(status, STATUS_ZERO_NORM);
-      const double d = sqrt(skk), dinv = 1.0 / d;
-      if (lane > k && lane < N) sO[k][lane] = cscale(sO[k][lane], dinv);
-      if (lane == 0) {
-        sO[k][k] = make_double2(d, 0.0);
-        sDinv[k] = make_double2(dinv, 0.0);
+  // ---- panels
+#pragma unroll 1
+  for (int kb = 0; kb < NT; ++kb) {
+    if (warp == kb % S::WARPS) {
+      double2 a[8];
+      const int row = min(lane, S::NP - 1);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = sm.O[row * S::LDO + 8 * kb + j];
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        const int k = 8 * kb + jj;
+        const double skk = __shfl_sync(0xffffffffu, a[jj].x, k < S::NP ? k : 0);
+        double d = 0.0, dinv = 0.0;
+        if (k < N) {
+          if (!(skk > 0.0)) flag(status, STATUS_ZERO_NORM);
+          d = sqrt(skk);
+          dinv = 1.0 / d;
+        }
+        if (lane == 0) sm.diag[k] = d;
+        // column k of L: rows below k (and the diagonal)
+        a[jj] = lane > k ? cscale(a[jj], dinv) : lane == k ? make_double2(d, 0.0) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int j = jj + 1; j < 8; ++j) {
+          const double2 lj = shfl2(a[jj], 8 * kb + j);
+          a[j] = csub(a[j], cmul(a[jj], conj_(lj)));
+        }
+      }
+      if (lane < S::NP)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sm.P[lane * S::LDP + j] = a[j];
+      __syncwarp();
+      // D = L_KK^-1: lane c solves column c by forward substitution
+      if (lane < 8) {
+        double2 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          double2 acc = make_double2(i == lane ? 1.0 : 0.0, 0.0);
+#pragma unroll
+          for (int p = 0; p < i; ++p) acc = csub(acc, cmul(sm.P[(8 * kb + i) * S::LDP + p], x[p]));
+          const double d = sm.P[(8 * kb + i) * S::LDP + i].x;
+          x[i] = d != 0.0 ? make_double2(acc.x / d, acc.y / d) : make_double2(0.0, 0.0);
+          sm.D[i * S::LDP + lane] = x[i];
+        }
       }
     }
     __syncthreads();
-    // S_ij -= conj(R_ki) R_kj for k < i <= j (loads first, as in the Gauss-Jordan update)
-    if (uj > k && uj < N) {
-      const double2 rkj = sO[k][uj];
-      double2 a[8], f[8];
+    // W[K, J] <- D W[K, J] (J < K), W[K, K] = D;  S[I, J] -= L[I, K] L[J, K]^H (I >= J > K)
+    for (int u = warp; u < S::UNITS; u += S::WARPS) {
+      int I, J;
+      lower_tile(u, I, J);
+      double2* c = sm.O + (8 * I + g) * S::LDO + 8 * J + 2 * t;
+      if (I == kb) {
+        double2 v0, v1;
+        if (J == kb) {
+          v0 = sm.D[g * S::LDP + 2 * t];
+          v1 = sm.D[g * S::LDP + 2 * t + 1];
+        } else {
+          double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = ui + 4 * r;
-        a[r] = sO[i][uj];
-        f[r] = sO[k][i];
-      }
+          for (int h = 0; h < 8; h += 4)
+            cmma(re, im, sm.D[g * S::LDP + h + t], sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g]);
+          v0 = make_double2(re[0], im[0]);
+          v1 = make_double2(re[1], im[1]);
+        }
+        __syncwarp();  // the tile is read by the warp that rewrites it
+        c[0] = v0;
+        c[1] = v1;
+      } else if (J > kb) {
+        const double2 c0 = c[0], c1 = c[1];
+        double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y};
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = ui + 4 * r;
-        if (i > k && i <= uj) sO[i][uj] = csub(a[r], cmulc(f[r], rkj));
+        for (int h = 0; h < 8; h += 4) {
+          const double2 l = sm.P[(8 * I + g) * S::LDP + h + t];
+          cmma(re, im, make_double2(-l.x, -l.y), conj_(sm.P[(8 * J + g) * S::LDP + h + t]));
+        }
+        c[0] = make_double2(re[0], im[0]);
+        c[1] = make_double2(re[1], im[1]);
       }
+    }
+    __syncthreads();
+    // W[I, J] -= L[I, K] W[K, J] (I > K, J <= K; W[I, K] was zero)
+    for (int u = warp; u < S::UNITS; u += S::WARPS) {
+      int I, J;
+      lower_tile(u, I, J);
+      if (I <= kb || J > kb) continue;
+      double2* c = sm.O + (8 * I + g) * S::LDO + 8 * J + 2 * t;
+      double2 c0 = make_double2(0.0, 0.0), c1 = c0;
+      if (J < kb) {
+        c0 = c[0];
+        c1 = c[1];
+      }
+      double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y};
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {
+        const double2 l = sm.P[(8 * I + g) * S::LDP + h + t];
+        cmma(re, im, make_double2(-l.x, -l.y), sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g]);
+      }
+      c[0] = make_double2(re[0], im[0]);
+      c[1] = make_double2(re[1], im[1]);
     }
     __syncthreads();
   }
-  double logsum = 0.0;
   if (tid < 32) {
-    // ---- X = R^-1 (upper): lane i, row i: X_ii = 1 / R_ii, X_ij = -(sum_{i<=k<j} X_ik R_kj) / R_jj
-    double2 x[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < j; ++k) {
-        const double2 rkj = sO[k][j];  // the same for every lane: a broadcast
-        acc.x += x[k].x * rkj.x - x[k].y * rkj.y;
-        acc.y += x[k].x * rkj.y + x[k].y * rkj.x;
-      }
-      const double di = j < N ? sDinv[j].x : 0.0;
-      x[j] = lane == j ? make_double2(di, 0.0) : (lane < j ? make_double2(-acc.x * di, -acc.y * di)
-                                                           : make_double2(0.0, 0.0));
-    }
-    // X_ij (i < j) to sO[j][i], below the diagonal: R is no longer read after the barrier
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (lane < j && j < N) sO[j][lane] = x[j];
-    double rmax = 0.0, rmin = 1.0e300;
+    double ls = 0.0, rmax = 0.0, rmin = 1.0e300;
     if (lane < N) {
-      const double r = sO[lane][lane].x;
-      logsum = log(r);
+      const double r = sm.diag[lane];
+      ls = log(r);
       rmax = rmin = r;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      logsum += __shfl_xor_sync(0xffffffffu, logsum, o);
+      ls += __shfl_xor_sync(0xffffffffu, ls, o);
       rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
       rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
     }
-    if (lane == 0) *sSpread = rmax / rmin;  // a lower bound on cond(phi); NaN when a pivot failed
+    if (lane == 0) {
+      sm.logsum = ls;
+      sm.spread = ls == ls ? rmax / rmin : ls;  // a lower bound on cond(phi); NaN when a pivot failed
+    }
   }
-  __syncthreads();
-  // ---- phi <- phi X: lane i = column i, rows m0 + 4 warp + a
-  const int nch = (M + 15) / 16;
+  // ---- phi <- phi W^H: out[m, j] = sum_{c <= j} phi[m, c] conj(W[j, c])
+  const int nch = (M + S::XM - 1) / S::XM;
   auto issue = [&](int ch) {
     if (ch < nch) {
-      double2* st = sStage + (ch % kORing) * kOStage;
-#pragma unroll
-      for (int u = 0; u < 16 * 32 / kThreads; ++u) {
-        const int e = tid + u * kThreads, r = e >> 5, c = e & 31, m = ch * 16 + r;
+      double2* st = sm.stage + (ch % S::XRING) * S::XSTAGE;
+      for (int e = tid; e < S::XM * S::NP; e += S::THREADS) {
+        const int r = e / S::NP, c = e % S::NP, m = ch * S::XM + r;
         const bool in = m < M && c < N;
-        cp_async16(st + e, phi + (in ? (size_t)m * N + c : 0), in ? 16 : 0);
+        cp_async16(st + r * S::LDX + c, phi + (in ? (size_t)m * N + c : 0), in ? 16 : 0);
       }
     }
     cp_async_commit();
   };
   issue(0);
-  issue(1);
+  if (S::XRING == 3) issue(1);
+  const int col = 4 * (g & 1) + (g >> 1);  // output column behind MMA column g (neighbouring stores)
   for (int ch = 0; ch < nch; ++ch) {
-    cp_async_wait<1>();
+    if (S::XRING == 3)
+      cp_async_wait<1>();
+    else
+      cp_async_wait<0>();
     __syncthreads();
-    issue(ch + 2);  // rows ahead of the ones rewritten below
-    const double2(*sPhi)[32] = reinterpret_cast<const double2(*)[32]>(sStage + (ch % kORing) * kOStage);
-    double2 acc[4];
+    issue(ch + S::XRING - 1);  // rows ahead of the ones rewritten below
+    const double2* a = sm.stage + (ch % S::XRING) * S::XSTAGE + (8 * warp + g) * S::LDX + t;
+    const int m = ch * S::XM + 8 * warp + g;
+    if (ch * S::XM + 8 * warp >= M) continue;
+    double2 av[2 * NT];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) acc[a] = make_double2(0.0, 0.0);
-#pragma unroll 8
-    for (int r = 0; r < 32; ++r) {
-      // X[r][lane]: below the diagonal of sO transposed, the diagonal in sDinv, zero for r > lane
-      const double2 xr = r < lane ? sO[lane][r] : (r == lane && r < N ? sDinv[r] : make_double2(0.0, 0.0));
+    for (int k = 0; k < 2 * NT; ++k) av[k] = a[4 * k];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const double2 p = sPhi[4 * warp + a][r];
-        acc[a].x += p.x * xr.x - p.y * xr.y;
-        acc[a].y += p.x * xr.y + p.y * xr.x;
+    for (int J = 0; J < NT; ++J) {
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+      const double2* w = sm.O + (8 * J + col) * S::LDO + t;
+#pragma unroll
+      for (int k = 0; k < 2 * (J + 1); ++k) cmma(re, im, av[k], conj_(w[4 * k]));
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = 8 * J + 4 * q + t;
+        if (m < M && j < N) phi[(size_t)m * N + j] = make_double2(re[q], im[q]);
       }
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int m = ch * 16 + 4 * warp + a;
-      if (m < M && lane < N) phi[(size_t)m * N + lane] = acc[a];
     }
   }
   cp_async_wait<0>();
   __syncthreads();
-  return logsum;  // valid in warp 0
+  return sm.logsum;
 }
 
 constexpr double kCholQR2 = 20.0;  // R-diagonal spread above which a block gets a second pass
@@ -606,16 +682,13 @@ constexpr double kCholQR2 = 20.0;  // R-diagonal spread above which a block gets
 // One CTA per walker: both spin blocks (the alpha block once when phib aliases it), then
 // detR = exp(sum log R_kk - detR_shift), log_detR += log detR, ovlp /= detR (the contract of
 // reortho_kernel in walkers.cu, which keeps N > 32).
-__global__ void __launch_bounds__(kThreads, 4) reortho_chol32_kernel(double2* __restrict__ phia,
-                                                                     double2* __restrict__ phib, int M, int na,
-                                                                     int nb, const double* __restrict__ detR_shift,
-                                                                     double* __restrict__ detR,
-                                                                     double* __restrict__ log_detR,
-                                                                     double2* __restrict__ ovlp, unsigned* status) {
-  __shared__ double2 sO[32][kNP];
-  __shared__ __align__(16) double2 sStage[kStage];
-  __shared__ double2 sDinv[32];
-  __shared__ double sSpread;
+template <int NT>
+__global__ void __launch_bounds__(RoShape<NT>::THREADS, 4)
+    reortho_chol32_kernel(double2* __restrict__ phia, double2* __restrict__ phib, int M, int na, int nb,
+                          const double* __restrict__ detR_shift, double* __restrict__ detR,
+                          double* __restrict__ log_detR, double2* __restrict__ ovlp, unsigned* status) {
+  extern __shared__ __align__(16) unsigned char gf_sm[];
+  RoShared<NT>& sm = *reinterpret_cast<RoShared<NT>*>(gf_sm);
   const int w = blockIdx.x;
   const bool alias = (phib == phia) && (nb == na);
   double logsum = 0.0, log_a = 0.0;
@@ -627,13 +700,17 @@ __global__ void __launch_bounds__(kThreads, 4) reortho_chol32_kernel(double2* __
       continue;
     }
     double2* phi = (s == 0 ? phia : phib) + (size_t)w * M * N;
-    double l = cholqr_block(phi, M, N, sO, sStage, sDinv, &sSpread, status);
+    double l = cholqr_block<NT>(phi, M, N, sm, status);
     // CholQR2: a second pass over the (now nearly orthonormal) result when R's diagonal spreads
     // by more than kCholQR2 (the first pass's error grows like cond(phi)^2 eps); R = R2 R1, so
     // the log-determinants add
-    if (!(sSpread <= kCholQR2)) l += cholqr_block(phi, M, N, sO, sStage, sDinv, &sSpread, status);
+    if (!(sm.spread <= kCholQR2)) {
+      __syncthreads();  // everyone has read the spread and the sum
+      l += cholqr_block<NT>(phi, M, N, sm, status);
+    }
     logsum += l;
     if (s == 0) log_a = l;
+    __syncthreads();
   }
   if (threadIdx.x == 0) {
     const double d = exp(logsum - detR_shift[w]);
@@ -641,6 +718,18 @@ __global__ void __launch_bounds__(kThreads, 4) reortho_chol32_kernel(double2* __
     log_detR[w] += log(d);
     ovlp[w] = cscale(ovlp[w], 1.0 / d);
   }
+}
+
+template <int NT>
+cudaError_t launch_reortho_nt(double2* phia, double2* phib, int W, int M, int na, int nb, const double* detR_shift,
+                              double* detR, double* log_detR, double2* ovlp, unsigned* status, cudaStream_t st) {
+  const int smem = (int)sizeof(RoShared<NT>);
+  auto k = reortho_chol32_kernel<NT>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k<<<W, RoShape<NT>::THREADS, smem, st>>>(phia, phib, M, na, nb, detR_shift, detR, log_detR, ovlp, status);
+  note_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -663,9 +752,12 @@ cudaError_t launch_reortho_chol32(double2* phia, double2* phib, int W, int M, in
                                   const double* detR_shift, double* detR, double* log_detR, double2* ovlp,
                                   unsigned* status, cudaStream_t st) {
   if (na < 1 || na > 32 || nb < 0 || nb > 32 || M <= 0 || W <= 0) return cudaErrorInvalidValue;
-  reortho_chol32_kernel<<<W, kThreads, 0, st>>>(phia, phib, M, na, nb, detR_shift, detR, log_detR, ovlp, status);
-  note_launch();
-  return cudaGetLastError();
+  switch ((max(na, nb) + 7) / 8) {
+    case 1: return launch_reortho_nt<1>(phia, phib, W, M, na, nb, detR_shift, detR, log_detR, ovlp, status, st);
+    case 2: return launch_reortho_nt<2>(phia, phib, W, M, na, nb, detR_shift, detR, log_detR, ovlp, status, st);
+    case 3: return launch_reortho_nt<3>(phia, phib, W, M, na, nb, detR_shift, detR, log_detR, ovlp, status, st);
+    default: return launch_reortho_nt<4>(phia, phib, W, M, na, nb, detR_shift, detR, log_detR, ovlp, status, st);
+  }
 }
 
 }  // namespace ipie_b200
