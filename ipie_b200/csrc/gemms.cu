@@ -250,7 +250,7 @@ using ExTall = RcCfg<96, 48, 4, 2, 2>;
 
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, C::OCC)
-    exchange_kernel(const __grid_constant__ RcOperands op, int W, int X, int N, int XB, int WB,
+    exchange_kernel(const __grid_constant__ RcOperands op, int W, int X, int N, int XB, int WB, int rows,
                     double2* __restrict__ part) {
   extern __shared__ __align__(16) double rc_sm[];
   constexpr int LDC = C::BN + 2;  // T_ij at stride LDC + 1 over i: odd, conflict-free
@@ -289,11 +289,14 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC)
     s = block_sum2(s, red);
     if (tid == 0) part[(size_t)blockIdx.y * W + w0 + wl] = s;
   }
+  if (blockIdx.y == gridDim.y - 1)
+    for (int e = tid; e < (rows - (int)gridDim.y) * wn; e += C::THREADS)
+      part[(size_t)((int)gridDim.y + e / wn) * W + w0 + e % wn] = make_double2(0.0, 0.0);
 }
 
 template <class C>
-static cudaError_t exchange_cfg(const double* rchol, const double2* ghalf, int W, int X, int M, int N, double2* part,
-                                cudaStream_t st) {
+static cudaError_t exchange_cfg(const double* rchol, const double2* ghalf, int W, int X, int M, int N, int rows,
+                                double2* part, cudaStream_t st) {
   const int XB = C::BM / N, WB = C::BN / N;
   const size_t need = sizeof(double2) * C::BM * (C::BN + 2), smem = need > C::SMEM ? need : C::SMEM;
   auto kern = exchange_kernel<C>;
@@ -305,16 +308,18 @@ static cudaError_t exchange_cfg(const double* rchol, const double2* ghalf, int W
   op.chunks = (M + kRcBK - 1) / kRcBK;
   op.vec_a = M % 2 == 0 && reinterpret_cast<uintptr_t>(rchol) % 16 == 0;
   op.vec_b = reinterpret_cast<uintptr_t>(ghalf) % 16 == 0;
-  kern<<<dim3((W + WB - 1) / WB, (X + XB - 1) / XB), C::THREADS, smem, st>>>(op, W, X, N, XB, WB, part);
+  kern<<<dim3((W + WB - 1) / WB, (X + XB - 1) / XB), C::THREADS, smem, st>>>(op, W, X, N, XB, WB, rows, part);
   note_launch();
   return cudaGetLastError();
 }
 
-// The shape whose rows and columns N fills better, among those that need no more partial rows than
-// the N rounded up to 8, 16 or 32 takes in 128 (callers size fixed buffers by that count).
+// Partial rows that callers provide and sum: one per 128 rows of N rounded up to 8, 16 or 32 (the last
+// row tile zeroes those that packing leaves over).
+static int exchange_row_vectors(int N) { return 128 / (N <= 8 ? 8 : N <= 16 ? 16 : 32); }
+
+// The shape whose rows and columns N fills better, among those that need no more partial rows.
 static bool exchange_tall(int N) {
-  const int np = N <= 8 ? 8 : N <= 16 ? 16 : 32;
-  if (ExTall::BM / N < 128 / np) return false;
+  if (ExTall::BM / N < exchange_row_vectors(N)) return false;
   const int wide = (ExWide::BM / N * N) * (ExWide::BN / N * N) * (ExTall::BM * ExTall::BN);
   const int tall = (ExTall::BM / N * N) * (ExTall::BN / N * N) * (ExWide::BM * ExWide::BN);
   return tall > wide;
@@ -327,12 +332,11 @@ cudaError_t launch_exchange(const double* rchol, const double2* ghalf, int W, in
     return cudaSuccess;
   }
   if (N > 32) return cudaErrorInvalidValue;
-  const bool tall = exchange_tall(N);
-  const int XB = (tall ? ExTall::BM : ExWide::BM) / N;
-  *ntiles = (X + XB - 1) / XB;
+  const int vectors = exchange_row_vectors(N);
+  *ntiles = (X + vectors - 1) / vectors;
   if (part == nullptr) return cudaSuccess;
-  return tall ? exchange_cfg<ExTall>(rchol, ghalf, W, X, M, N, part, st)
-              : exchange_cfg<ExWide>(rchol, ghalf, W, X, M, N, part, st);
+  return exchange_tall(N) ? exchange_cfg<ExTall>(rchol, ghalf, W, X, M, N, *ntiles, part, st)
+                          : exchange_cfg<ExWide>(rchol, ghalf, W, X, M, N, *ntiles, part, st);
 }
 
 }  // namespace ipie_b200
