@@ -1,7 +1,9 @@
 // Green's function, overlap and reorthogonalisation for spin blocks of N <= 32 electrons: one CTA of
-// 96 or 128 threads per walker, four per SM, on the f64 tensor cores.
+// 96 or 128 threads per walker and distinct spin block, four per SM, on the f64 tensor cores.
 // ovlp_w = prod_s phase_s * exp(sum_s log|det O_s| - log_shift_w).
 // Same contracts as gf_overlap_kernel and reortho_kernel (walkers.cu), which keep N > 32.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -30,7 +32,9 @@ constexpr int kChunk = 8;  // rows of phi / psi* per shared-memory chunk of the 
 //       loads free of bank conflicts.
 // The floor is the f64 tensor pipe's time for the two products (28k cycles per SM and walker at
 // M = 200, N = 32).  2048 walkers, M = 200, N = 32: 535 -> 354 us; 512, M = 76, N = 10: 46 -> 19 us; 777, M =
-// 149, N = 23 + 17: 280 -> 175 us (against DFMA products and the column by column elimination).
+// 149, N = 23 + 17: 280 -> 175 us (against DFMA products and the column by column elimination), and 175 ->
+// 151 us with a CTA per spin instead of both in one (640, M = 108, N = 15 + 15: 89 -> 72 us): the pivot chains of
+// the two spins run side by side and the last round of CTAs is shorter.
 template <int NT>
 struct GfShape {
   static constexpr int WARPS = NT == 3 ? 3 : 4, THREADS = 32 * WARPS, NP = 8 * NT;
@@ -336,45 +340,66 @@ __global__ void __launch_bounds__(GfShape<NT>::THREADS, 4)
     gf_mma_kernel(const double2* __restrict__ phia, const double2* __restrict__ phib, int M, int na, int nb,
                   const double2* __restrict__ psia_c, const double2* __restrict__ psib_c,
                   const double* __restrict__ log_shift, double2* __restrict__ ghalfa, double2* __restrict__ ghalfb,
-                  double2* __restrict__ ovlp, double2* __restrict__ logdet, unsigned* status) {
+                  double2* __restrict__ ovlp, double2* __restrict__ logdet, unsigned* status, int S) {
   extern __shared__ __align__(16) unsigned char gf_sm[];
   GfShared<NT>& sm = *reinterpret_cast<GfShared<NT>*>(gf_sm);
-  const int w = blockIdx.x;
-  // spin aliasing: phib == phia with nb == na is one block counted twice
-  const bool alias = (phib == phia) && (nb == na);
-  double logsum = 0.0;
-  double2 phase = make_double2(1.0, 0.0);  // (thread 0's are used)
-  for (int s = 0; s < 2; ++s) {
-    const int N = s == 0 ? na : nb;
-    if (N == 0) continue;
-    if (s == 1 && alias) {
-      logsum += logsum;
-      phase = cmul(phase, phase);
-      if (logdet != nullptr && threadIdx.x == 0) logdet[(size_t)w * 2 + 1] = logdet[(size_t)w * 2];
-      continue;
-    }
-    const double2* phi = (s == 0 ? phia : phib) + (size_t)w * M * N;
-    gf_overlap_tiles<NT>(phi, s == 0 ? psia_c : psib_c, M, N, sm);
-    __syncthreads();
-    gf_invert<NT>(N, sm, status);
-    gf_determinant<NT>(N, sm);
-    if (threadIdx.x == 0) {
-      logsum += sm.red[0].x;
-      phase = cmul(phase, sm.red[1]);
-      if (logdet != nullptr) logdet[(size_t)w * 2 + s] = make_double2(sm.red[0].x, atan2(sm.red[1].y, sm.red[1].x));
-    }
-    if (WITH_GHALF) {
-      double2* g1 = (s == 0 ? ghalfa : ghalfb) + (size_t)w * N * M;
-      double2* g2 = (s == 0 && alias && nb > 0 && ghalfb != ghalfa) ? ghalfb + (size_t)w * N * M : nullptr;
-      gf_ghalf<NT>(phi, M, N, sm, g1, g2);
-    }
-    __syncthreads();
+  // two distinct spin blocks: a cluster of two CTAs, one per spin (S = 2); one block, or one
+  // counted twice (phib == phia with nb == na): one CTA
+  const int w = blockIdx.x / S, s = blockIdx.x % S;
+  const bool alias = S == 1 && nb > 0 && na > 0;
+  const int N = S == 2 ? (s == 0 ? na : nb) : max(na, nb);
+  const bool beta = S == 2 ? s == 1 : na == 0;
+  const double2* phi = (beta ? phib : phia) + (size_t)w * M * N;
+  gf_overlap_tiles<NT>(phi, beta ? psib_c : psia_c, M, N, sm);
+  __syncthreads();
+  gf_invert<NT>(N, sm, status);
+  gf_determinant<NT>(N, sm);
+  if (threadIdx.x == 0 && logdet != nullptr) {
+    const double2 ld = make_double2(sm.red[0].x, atan2(sm.red[1].y, sm.red[1].x));
+    logdet[(size_t)w * 2 + (beta ? 1 : 0)] = ld;
+    if (alias) logdet[(size_t)w * 2 + 1] = ld;
   }
-  if (threadIdx.x == 0) {
+  if (S == 2) cooperative_groups::this_cluster().barrier_arrive();  // this spin's determinant is in place
+  if (WITH_GHALF) {
+    double2* g1 = (beta ? ghalfb : ghalfa) + (size_t)w * N * M;
+    double2* g2 = (alias && ghalfb != ghalfa) ? ghalfb + (size_t)w * N * M : nullptr;
+    gf_ghalf<NT>(phi, M, N, sm, g1, g2);
+  }
+  double logsum = sm.red[0].x;  // (thread 0 wrote them)
+  double2 phase = sm.red[1];
+  if (S == 2) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    cl.barrier_wait();
+    if (s == 0 && threadIdx.x == 0) {
+      const double2* other = cl.map_shared_rank(sm.red, 1);
+      logsum += other[0].x;
+      phase = cmul(phase, other[1]);
+    }
+    cl.sync();  // the peer stays until its determinant is read
+  } else if (alias) {
+    logsum += logsum;
+    phase = cmul(phase, phase);
+  }
+  if (s == 0 && threadIdx.x == 0) {
     const double2 o = cscale(phase, exp(logsum - log_shift[w]));
     if (!finite2(o)) flag(status, STATUS_NONFINITE);
     ovlp[w] = o;
   }
+}
+
+// grid and cluster of a kernel that gives each distinct spin block of a walker a CTA of its own
+static void spin_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int W, int S, int threads, int smem,
+                        cudaStream_t st) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3((unsigned)(W * S));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)S;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
 }
 
 template <int NT>
@@ -385,8 +410,13 @@ cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M
   auto k = ghalfa != nullptr ? gf_mma_kernel<NT, true> : gf_mma_kernel<NT, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k<<<W, GfShape<NT>::THREADS, smem, st>>>(phia, phib, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb, ovlp,
-                                           logdet, status);
+  const int S = na > 0 && nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  spin_config(cfg, attr, W, S, GfShape<NT>::THREADS, smem, st);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, k, phia, phib, M, na, nb, psia_c, psib_c, log_shift, ghalfa, ghalfb,
+                                            ovlp, logdet, status, S);
+  if (le != cudaSuccess) return le;
   note_launch();
   return cudaGetLastError();
 }
@@ -679,41 +709,39 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
 
 constexpr double kCholQR2 = 20.0;  // R-diagonal spread above which a block gets a second pass
 
-// One CTA per walker: both spin blocks (the alpha block once when phib aliases it), then
 // detR = exp(sum log R_kk - detR_shift), log_detR += log detR, ovlp /= detR (the contract of
 // reortho_kernel in walkers.cu, which keeps N > 32).
 template <int NT>
 __global__ void __launch_bounds__(RoShape<NT>::THREADS, 4)
     reortho_chol32_kernel(double2* __restrict__ phia, double2* __restrict__ phib, int M, int na, int nb,
                           const double* __restrict__ detR_shift, double* __restrict__ detR,
-                          double* __restrict__ log_detR, double2* __restrict__ ovlp, unsigned* status) {
+                          double* __restrict__ log_detR, double2* __restrict__ ovlp, unsigned* status, int S) {
   extern __shared__ __align__(16) unsigned char gf_sm[];
   RoShared<NT>& sm = *reinterpret_cast<RoShared<NT>*>(gf_sm);
-  const int w = blockIdx.x;
-  const bool alias = (phib == phia) && (nb == na);
-  double logsum = 0.0, log_a = 0.0;
-  for (int s = 0; s < 2; ++s) {
-    const int N = s == 0 ? na : nb;
-    if (N == 0) continue;
-    if (s == 1 && alias) {
-      logsum += log_a;
-      continue;
-    }
-    double2* phi = (s == 0 ? phia : phib) + (size_t)w * M * N;
-    double l = cholqr_block<NT>(phi, M, N, sm, status);
-    // CholQR2: a second pass over the (now nearly orthonormal) result when R's diagonal spreads
-    // by more than kCholQR2 (the first pass's error grows like cond(phi)^2 eps); R = R2 R1, so
-    // the log-determinants add
-    if (!(sm.spread <= kCholQR2)) {
-      __syncthreads();  // everyone has read the spread and the sum
-      l += cholqr_block<NT>(phi, M, N, sm, status);
-    }
-    logsum += l;
-    if (s == 0) log_a = l;
-    __syncthreads();
+  // as the Green's function: one CTA per distinct spin block, a walker's two in a cluster
+  const int w = blockIdx.x / S, s = blockIdx.x % S;
+  const bool alias = S == 1 && nb > 0 && na > 0;
+  const int N = S == 2 ? (s == 0 ? na : nb) : max(na, nb);
+  double2* phi = ((S == 2 ? s == 1 : na == 0) ? phib : phia) + (size_t)w * M * N;
+  double l = cholqr_block<NT>(phi, M, N, sm, status);
+  // CholQR2: a second pass over the (now nearly orthonormal) result when R's diagonal spreads
+  // by more than kCholQR2 (the first pass's error grows like cond(phi)^2 eps); R = R2 R1, so
+  // the log-determinants add
+  if (!(sm.spread <= kCholQR2)) {
+    __syncthreads();  // everyone has read the spread and the sum
+    l += cholqr_block<NT>(phi, M, N, sm, status);
   }
-  if (threadIdx.x == 0) {
-    const double d = exp(logsum - detR_shift[w]);
+  if (S == 2) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (threadIdx.x == 0) sm.logsum = l;
+    cl.sync();
+    if (s == 0 && threadIdx.x == 0) l += *cl.map_shared_rank(&sm.logsum, 1);
+    cl.sync();  // the peer stays until its sum is read
+  } else if (alias) {
+    l += l;
+  }
+  if (s == 0 && threadIdx.x == 0) {
+    const double d = exp(l - detR_shift[w]);
     detR[w] = d;
     log_detR[w] += log(d);
     ovlp[w] = cscale(ovlp[w], 1.0 / d);
@@ -727,7 +755,13 @@ cudaError_t launch_reortho_nt(double2* phia, double2* phib, int W, int M, int na
   auto k = reortho_chol32_kernel<NT>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k<<<W, RoShape<NT>::THREADS, smem, st>>>(phia, phib, M, na, nb, detR_shift, detR, log_detR, ovlp, status);
+  const int S = na > 0 && nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  spin_config(cfg, attr, W, S, RoShape<NT>::THREADS, smem, st);
+  const cudaError_t le =
+      cudaLaunchKernelEx(&cfg, k, phia, phib, M, na, nb, detR_shift, detR, log_detR, ovlp, status, S);
+  if (le != cudaSuccess) return le;
   note_launch();
   return cudaGetLastError();
 }
