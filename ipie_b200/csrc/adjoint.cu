@@ -71,7 +71,8 @@ __global__ void rotate_onebody_kernel(const double2* __restrict__ psi_c, const d
 // L entry read is 8 R operations, so the bound is the f64 tensor pipe.  Few walkers: the x range
 // is split over a cluster of S CTAs whose accumulators are added through distributed shared memory
 // in rank order.  512 walkers, M = 76, N = 10, X = 400, one spin: 6.91 ms as scalar products from
-// shared memory, 0.70 ms here (17.7 TFLOP/s; the tensor pipe's peak is 36.9).
+// shared memory, 0.64 ms here (19.4 TFLOP/s; the tensor pipe's peak is 36.9; 0.70 ms with blocks of 40
+// Cholesky rows instead of 80, X_wx read from global memory and the index divisions in the loop).
 constexpr int kVjWarps = 16;
 constexpr int kVjThreads = 32 * kVjWarps;
 constexpr int kVjMaxUnits = 8;  // 8 x 8 accumulator tiles per warp (4 doubles per lane each)
@@ -104,15 +105,16 @@ static bool vjp_shape(int W, int X, int M, int N, VjpShape& best) {
     s.RT = (s.R + 7) / 8;
     s.units = (s.RT * s.CT2 + kVjWarps - 1) / kVjWarps;
     if (s.RT > 5 || s.units > kVjMaxUnits) break;
-    // blocks of up to 40 Cholesky rows, double buffered, where shared memory holds them
+    // blocks of up to 80 Cholesky rows, double buffered, where shared memory holds them
     bool fits = false;
     for (s.nbuf = 2; s.nbuf >= 1 && !fits; --s.nbuf) {
-      for (s.XB = N >= 40 ? 1 : 40 / N; s.XB >= 1 && !fits; --s.XB) {
+      for (s.XB = 80 / N; s.XB >= 1 && !fits; --s.XB) {
         s.KB = s.XB * N;
         s.CT1 = (s.KB + 7) / 8;
         s.KB4 = (s.KB + 3) & ~3;
         s.ldq = stride4(s.KB4, 8);
-        s.smem = sizeof(double2) * ((size_t)s.RT * 8 * (s.ldg + s.ldq)) + sizeof(double) * s.nbuf * s.CT1 * 8 * s.ldl;
+        s.smem = sizeof(double2) * ((size_t)s.RT * 8 * (s.ldg + s.ldq) + 2 * s.WB * s.XB) +
+                 sizeof(double) * s.nbuf * s.CT1 * 8 * s.ldl + sizeof(int) * 3 * (s.R + s.KB);
         fits = s.smem <= 232448;
         if (fits) break;
       }
@@ -145,15 +147,31 @@ __global__ void __launch_bounds__(kVjThreads, 1)
   extern __shared__ __align__(16) unsigned char vjp_sm[];
   double2* const sG = reinterpret_cast<double2*>(vjp_sm);  // (8 RT, ldg)
   double2* const sQ = sG + s.RT * 8 * s.ldg;               // (8 RT, ldq)
-  double* const sL = reinterpret_cast<double*>(sQ + s.RT * 8 * s.ldq);  // nbuf x (8 CT1, ldl)
+  double2* const sX = sQ + s.RT * 8 * s.ldq;                // 2 x (WB, XB): X_wx of a block
+  double* const sL = reinterpret_cast<double*>(sX + 2 * s.WB * s.XB);  // nbuf x (8 CT1, ldl)
+  int* const tr = reinterpret_cast<int*>(sL + s.nbuf * s.CT1 * 8 * s.ldl);  // rows of S: place in Q, w, i
+  int* const tc = tr + 3 * s.R;                                             // columns of S: place in Q, x, j
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int w0 = (int)(blockIdx.x / s.S) * s.WB, rank = (int)(blockIdx.x % s.S);
   const int lsize = s.CT1 * 8 * s.ldl;
   // zeros everywhere first: the padding rows and columns keep them
   for (int e = tid; e < s.RT * 8 * (s.ldg + s.ldq); e += kVjThreads) sG[e] = make_double2(0.0, 0.0);
   for (int e = tid; e < s.nbuf * lsize; e += kVjThreads) sL[e] = 0.0;
+  for (int r = tid; r < s.R; r += kVjThreads) {
+    const int wl = r / N, i = r - wl * N;
+    tr[r] = wl * N * s.ldq + i;
+    tr[s.R + r] = wl;
+    tr[2 * s.R + r] = i;
+  }
+  for (int c = tid; c < s.KB; c += kVjThreads) {
+    const int xl = c / N, j = c - xl * N;
+    tc[c] = j * s.ldq + xl * N;
+    tc[s.KB + c] = xl;
+    tc[2 * s.KB + c] = j;
+  }
   __syncthreads();
-  // Cholesky rows of block b (contiguous in rchol) into buffer `buf`, zeros for vectors past X
+  // Cholesky rows of block b (contiguous in rchol) into buffer `buf`, zeros for vectors past X, and
+  // its X_wx (zeros past X and W) into the buffer of b's parity
   auto load_block = [&](int b, int buf) {
     const long long row0 = (long long)b * s.KB, rows = (long long)X * N - row0;
     const double* src = rchol + row0 * M;
@@ -171,6 +189,11 @@ __global__ void __launch_bounds__(kVjThreads, 1)
         const bool in = r < rows;
         cp_async8(dst + r * s.ldl + c, in ? src + (size_t)r * M + c : rchol, in ? 8 : 0);
       }
+    }
+    for (int e = tid; e < s.WB * s.XB; e += kVjThreads) {
+      const int wl = e / s.XB, x = b * s.XB + e - wl * s.XB;
+      const bool in = x < X && w0 + wl < W;
+      cp_async16(sX + (b & 1) * s.WB * s.XB + e, in ? xv + (size_t)(w0 + wl) * X + x : xv, in ? 16 : 0);
     }
     cp_async_commit();
   };
@@ -225,19 +248,19 @@ __global__ void __launch_bounds__(kVjThreads, 1)
       }
       const int r = rt * 8 + g;
       if (r < s.R) {
-        const int wl = r / N, i = r - wl * N;
+        const int qr = tr[r], wl = tr[s.R + r], i = tr[2 * s.R + r];
+        const double2* cx = sX + (b & 1) * s.WB * s.XB + wl * s.XB;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const int c = ct * 8 + 2 * t + q;
           if (c < s.KB) {
-            const int xl = c / N, j = c - xl * N, x = b * s.XB + xl;
             double2 v = make_double2(-fx2 * (dr[0][q] + dr[1][q]), -fx2 * (di[0][q] + di[1][q]));
-            if (i == j && x < X && w0 + wl < W) {
-              const double2 cx = xv[(size_t)(w0 + wl) * X + x];
-              v.x += fc2 * cx.x;
-              v.y += fc2 * cx.y;
+            if (i == tc[2 * s.KB + c]) {
+              const double2 x = cx[tc[s.KB + c]];
+              v.x += fc2 * x.x;
+              v.y += fc2 * x.y;
             }
-            sQ[(wl * N + j) * s.ldq + xl * N + i] = v;
+            sQ[qr + tc[c]] = v;
           }
         }
       }

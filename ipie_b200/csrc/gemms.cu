@@ -242,7 +242,7 @@ cudaError_t launch_taylor(const double2* vhs, const double2* phi_in, double2* ph
 // is the one of two that N fills better.  The epilogue parks T in shared memory and sums each
 // (x, w) block's products over unordered pairs (i, j) into one partial per (tile row, walker); T
 // never reaches global memory.  At 2 CTAs per SM one's epilogue runs under the other's products.
-// UHF, 640 walkers, M = 108, N = 15, X = 600, one spin: 1.99 -> 1.69 ms (37.3 GFLOP: 22
+// UHF, 640 walkers, M = 108, N = 15, X = 600, one spin: 1.99 -> 1.67 ms (37.3 GFLOP: 22
 // TFLOP/s, 25 with the padding of 15 to 120 / 8 rows); 512 walkers, M = 76, N = 10, X = 400: 0.78 -> 0.34 ms.
 // ---------------------------------------------------------------------------
 using ExWide = RcCfg<128, 32, 4, 2, 2>;
@@ -272,22 +272,37 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC)
     }
   __syncthreads();
   // unordered pairs of {0..N-1} as (i, i + d mod N), d = 0 .. N/2: once each, except that d = N/2
-  // of an even N meets every pair twice
-  __shared__ double2 red[32];
-  const int nd = N / 2 + 1, xn = min(XB, X - x0), wn = min(WB, W - w0);
-  for (int wl = 0; wl < wn; ++wl) {
-    double2 s = make_double2(0.0, 0.0);
-    for (int e = tid; e < xn * nd * N; e += C::THREADS) {
-      const int q = e / N, i = e - q * N, xl = q / nd, d = q - xl * nd;
-      const int j = i + d < N ? i + d : i + d - N;
-      const double2* blk = sT + xl * N * LDC + wl * N;
+  // of an even N meets every pair twice.  A warp takes consecutive (w, x) blocks, so it crosses few
+  // walkers and reduces once per walker it meets.
+  constexpr int NW = C::THREADS / 32;
+  __shared__ double2 red[C::BN][NW];
+  const int xn = min(XB, X - x0), wn = min(WB, W - w0), pairs = (N / 2 + 1) * N;
+  for (int e = tid; e < wn * NW; e += C::THREADS) red[e / NW][e % NW] = make_double2(0.0, 0.0);
+  __syncthreads();
+  const int b0 = xn * wn * warp / NW, b1 = xn * wn * (warp + 1) / NW;
+  double2 s = make_double2(0.0, 0.0);
+  for (int b = b0; b < b1; ++b) {
+    const int wl = b / xn, xl = b - wl * xn;
+    const double2* blk = sT + xl * N * LDC + wl * N;
+    for (int e = lane; e < pairs; e += 32) {
+      const int d = e / N, i = e - d * N, j = i + d < N ? i + d : i + d - N;
       const double2 p = cmul(blk[i * LDC + j], blk[j * LDC + i]);
       const double f = (d == 0 || 2 * d == N) ? 1.0 : 2.0;
       s.x += f * p.x;
       s.y += f * p.y;
     }
-    s = block_sum2(s, red);
-    if (tid == 0) part[(size_t)blockIdx.y * W + w0 + wl] = s;
+    if (b + 1 == b1 || xl == xn - 1) {
+      s = warp_sum2(s);
+      if (lane == 0) red[wl][warp] = s;
+      s = make_double2(0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  if (tid < wn) {
+    double2 v = red[tid][0];
+#pragma unroll
+    for (int q = 1; q < NW; ++q) v = cadd(v, red[tid][q]);
+    part[(size_t)blockIdx.y * W + w0 + tid] = v;
   }
   if (blockIdx.y == gridDim.y - 1)
     for (int e = tid; e < (rows - (int)gridDim.y) * wn; e += C::THREADS)
