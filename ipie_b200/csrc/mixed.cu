@@ -7,6 +7,7 @@
 #include "../../include/ipie_b200.h"
 #include "../../include/ipie_b200_testing.h"
 #include "kernels.h"
+#include "exchange_f16.cuh"
 #include "umma_gemm.cuh"
 
 namespace ipie_b200 {
@@ -1049,8 +1050,47 @@ static cudaError_t exchange3_np(const void* r_hi, const void* r_lo, double rscal
                                                                  148);
 }
 
+static cudaError_t device_sms(int* sms) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
+template <int NP>
+static cudaError_t exchange_tmem_np(const void* r_hi, const void* r_lo, double rscale, const GPad& gp, int W, int X,
+                                    int M, double2* part, unsigned* status, cudaStream_t st) {
+  using S = ExTmemShape;
+  const int Mp = f16_ld(M);
+  if (W <= 0 || X <= 0) return cudaErrorInvalidValue;
+  if (((reinterpret_cast<uintptr_t>(gp.hi) | reinterpret_cast<uintptr_t>(gp.lo)) & 15) != 0) return cudaErrorInvalidValue;
+  GemmMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  cudaError_t e;
+  if ((e = map_f16_pair(&maps.b_hi, &maps.b_lo, r_hi, r_lo, (long long)X * NP, M, Mp, S::BN, false, &maps.b_planes)) !=
+      cudaSuccess)
+    return e;
+  int sms = 0;
+  if ((e = device_sms(&sms)) != cudaSuccess) return e;
+  auto kern = exchange_tmem_kernel<NP>;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES)) != cudaSuccess)
+    return e;
+  const ExRuns runs = exchange_tmem_runs(W, X, NP, sms);
+  kern<<<runs.g, S::THREADS, S::SMEM_BYTES, st>>>(maps, gp.hi, gp.lo, M, Mp, runs, W, 1.0 / (rscale * rscale), gp.scale,
+                                                  runs.rows(), part, status);
+  note_launch();
+  return cudaGetLastError();
+}
+
+// The walkers' rows stay in tensor memory up to M = 256 (two planes of 128 columns next to the two
+// accumulator buffers); longer rows stream both operands.
 static cudaError_t exchange3(const void* r_hi, const void* r_lo, double rscale, const GPad& gp, int W, int X, int M,
                              int N, double2* part, unsigned* status, cudaStream_t st) {
+  if (M <= ExTmemShape::MAX_K) switch (exchange_np(N)) {
+      case 8: return exchange_tmem_np<8>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
+      case 16: return exchange_tmem_np<16>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
+      case 32: return exchange_tmem_np<32>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
+      default: return cudaErrorInvalidValue;
+    }
   switch (exchange_np(N)) {
     case 8: return exchange3_np<8>(r_hi, r_lo, rscale, gp, W, X, M, N, part, status, st);
     case 16: return exchange3_np<16>(r_hi, r_lo, rscale, gp, W, X, M, N, part, status, st);
@@ -1059,7 +1099,13 @@ static cudaError_t exchange3(const void* r_hi, const void* r_lo, double rscale, 
   }
 }
 
-int exchange3_rows(int X, int N) { return (X * exchange_np(N) + kBM - 1) / kBM; }
+// Partial rows that exchange3 leaves: never more than the callers' ceil(X NP / 128) per walker.
+static int exchange3_rows(int W, int X, int M, int N) {
+  const int np = exchange_np(N);
+  int sms = 0;
+  if (M <= ExTmemShape::MAX_K && device_sms(&sms) == cudaSuccess) return exchange_tmem_runs(W, X, np, sms).rows();
+  return (X * np + kBM - 1) / kBM;
+}
 
 cudaError_t mixed_vhs(const void* cp_hi, const void* cp_lo, const int* ii, const int* jj, int P, int X, int M,
                       const void* xs_hi, const void* xs_lo, int W, double sqrt_dt, double cp_scale, int f16_planes,
@@ -1302,7 +1348,7 @@ extern "C" int ipie_b200_exchange_mixed(const void* r_hi, const void* r_lo, doub
   cudaError_t e = umma::pad_ghalf((CC)ghalf, W, M, N, NP, gp, st, delta ? (CC)ghalf_trial : nullptr);
   if (e == cudaSuccess) e = umma::exchange3(r_hi, r_lo, r_scale, gp, W, X, M, N, p, status, st);
   if (e != cudaSuccess) return (int)e;
-  int rows = umma::exchange3_rows(X, N);
+  int rows = umma::exchange3_rows(W, X, M, N);
   if (delta) {
     e = umma::exchange_ref_row((CC)ghalf, (CC)ghalf_trial, (CC)kmat, W, N * M, (CC)raw_trial, p + (size_t)rows * W, st);
     if (e != cudaSuccess) return (int)e;
@@ -1367,14 +1413,14 @@ extern "C" int ipie_b200_local_energy_mixed(int rhf, const double* rchola, const
     e = umma::coulomb3(ra_hi, ra_lo, ra_scale, gp, W, X, M, NPa, xv, 1, alias ? 2.0 : 1.0, status, st);
   if (e == cudaSuccess) e = umma::exchange3(ra_hi, ra_lo, ra_scale, gp, W, X, M, na, part, status, st);
   if (e != cudaSuccess) return (int)e;
-  int rows = umma::exchange3_rows(X, na);
+  int rows = umma::exchange3_rows(W, X, M, na);
   if (use_b) {
     e = umma::pad_ghalf((CC)ghalfb, W, M, nb, NPb, gp, st, delta ? (CC)ghalf_trial_b : nullptr);
     if (e == cudaSuccess && delta) e = umma::coulomb3(rb_hi, rb_lo, rb_scale, gp, W, X, M, NPb, xv, 1, 1.0, status, st);
     if (e == cudaSuccess)
       e = umma::exchange3(rb_hi, rb_lo, rb_scale, gp, W, X, M, nb, part + (size_t)rows * W, status, st);
     if (e != cudaSuccess) return (int)e;
-    rows += umma::exchange3_rows(X, nb);
+    rows += umma::exchange3_rows(W, X, M, nb);
   }
   if (delta) {
     e = umma::exchange_ref_row((CC)ghalfa, (CC)ghalf_trial_a, (CC)kmat_a, W, na * M, (CC)raw_trial,
