@@ -266,36 +266,39 @@ __global__ void __launch_bounds__(kVjThreads, 1)
       }
     }
     __syncthreads();
-    // acc += Q L
-    if (mine == U2) {
-      for (int k = 0; k < s.KB4; k += 4) {
-        const double* lk = l + k * s.ldl;
+    // acc += Q L, each block summed by itself first: one chain over all X N terms doubles the rounding error
+    if (mine > 0) {
+      double re[U2][2], im[U2][2];
 #pragma unroll
-        for (int u = 0; u < U2; ++u) {
-          const double2 a = sQ[arow[u] + k];
-          const double v = lk[bcol[u]];
-          double re[2] = {acc[u][0].x, acc[u][1].x}, im[2] = {acc[u][0].y, acc[u][1].y};
-          dmma884(re, a.x, v);
-          dmma884(im, a.y, v);
-          acc[u][0] = make_double2(re[0], im[0]);
-          acc[u][1] = make_double2(re[1], im[1]);
+      for (int u = 0; u < U2; ++u) re[u][0] = re[u][1] = im[u][0] = im[u][1] = 0.0;
+      if (mine == U2) {
+        for (int k = 0; k < s.KB4; k += 4) {
+          const double* lk = l + k * s.ldl;
+#pragma unroll
+          for (int u = 0; u < U2; ++u) {
+            const double2 a = sQ[arow[u] + k];
+            const double v = lk[bcol[u]];
+            dmma884(re[u], a.x, v);
+            dmma884(im[u], a.y, v);
+          }
+        }
+      } else {
+        for (int k = 0; k < s.KB4; k += 4) {
+          const double* lk = l + k * s.ldl;
+#pragma unroll
+          for (int u = 0; u < U2; ++u) {
+            if (u >= mine) break;
+            const double2 a = sQ[arow[u] + k];
+            const double v = lk[bcol[u]];
+            dmma884(re[u], a.x, v);
+            dmma884(im[u], a.y, v);
+          }
         }
       }
-    } else if (mine > 0) {
-      for (int k = 0; k < s.KB4; k += 4) {
-        const double* lk = l + k * s.ldl;
 #pragma unroll
-        for (int u = 0; u < U2; ++u) {
-          if (u >= mine) break;
-          const double2 a = sQ[arow[u] + k];
-          const double v = lk[bcol[u]];
-          double re[2] = {acc[u][0].x, acc[u][1].x}, im[2] = {acc[u][0].y, acc[u][1].y};
-          dmma884(re, a.x, v);
-          dmma884(im, a.y, v);
-          acc[u][0] = make_double2(re[0], im[0]);
-          acc[u][1] = make_double2(re[1], im[1]);
-        }
-      }
+      for (int u = 0; u < U2; ++u)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) acc[u][q] = cadd(acc[u][q], make_double2(re[u][q], im[u][q]));
     }
     if (s.nbuf == 1) {
       __syncthreads();  // the one buffer is free
