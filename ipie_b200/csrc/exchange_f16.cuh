@@ -35,13 +35,6 @@
 namespace ipie_b200 {
 namespace umma {
 
-// true in one lane of a converged warp, the same one each time
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r)::"memory");
-  return r != 0;
-}
-
 // 128 x N x 16 FP16 product with the left operand in tensor memory (row = lane, two K per column)
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
@@ -50,11 +43,6 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
           d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-
-// the same answer in every lane
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort, unsigned* status) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, status)) != 0;
 }
 
 struct ExTmemShape {

@@ -53,6 +53,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// mbar_wait by a whole converged warp: the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort, unsigned* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, status)) != 0;
+}
+
+// true in one lane of a converged warp, the same one each time
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r)::"memory");
+  return r != 0;
+}
+
 // ------------------------------------------------------------------ TMA
 // One thread issuing tensor (or bulk) copies sustains about one ring stage per ~900 SM cycles on
 // B200, whatever the box size up to 32 KB (measured: 16 KB boxes 18 B/clk per SM, 32 KB boxes

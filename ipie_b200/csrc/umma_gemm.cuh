@@ -23,7 +23,7 @@
 // the chunks (chunk_full / chunk_empty mbarriers) and run the epilogue on their
 // group's summed 128 values (a tile of BN = 256 is handed to the epilogue as two
 // 128-column tiles); then one warp whose lane 0 issues TMA loads into a
-// STAGES-deep ring (full/empty mbarriers) and one whose lane 0 issues
+// STAGES-deep ring (full/empty mbarriers) and one that issues
 // tcgen05.mma.  One-group epilogues may synchronise with bar.sync 1, 128
 // (epi_sync), never with __syncthreads.
 //
@@ -290,7 +290,9 @@ __global__ void __launch_bounds__(GemmRoles<NA, BN>::kThreads, 1)
     }
     __syncwarp();
   } else if (warp == R::kMmaWarp) {
-    if (lane == 0 && rank == 0) {
+    // the whole warp runs the loop and an elected lane issues, which keeps descriptors and addresses
+    // warp-uniform (from a lane-0 branch every product costs the issuing lane about 25 cycles more)
+    if (rank == 0) {
       constexpr uint32_t idesc = KIND != KIND_TF32 ? idesc_f16(kBM * CG, BN) : idesc_tf32(kBM, BN);
       uint32_t g = 0, c = 0;  // stage uses and chunks so far (all tiles)
       bool ok = true;
@@ -299,12 +301,12 @@ __global__ void __launch_bounds__(GemmRoles<NA, BN>::kThreads, 1)
           const bool first = (kb % CKB) == 0;
           const bool last = (kb % CKB) == CKB - 1 || kb == nk - 1;
           const uint32_t buf = c & 1;
-          if (first && c >= 2 && !mbar_wait(&cempty[buf], ((c >> 1) - 1) & 1, abort_flag, status)) {
+          if (first && c >= 2 && !mbar_wait_warp(&cempty[buf], ((c >> 1) - 1) & 1, abort_flag, status)) {
             ok = false;
             break;
           }
           const uint32_t s = g % STAGES, r = g / STAGES;
-          if (!mbar_wait(&full[s], r & 1, abort_flag, status)) {
+          if (!mbar_wait_warp(&full[s], r & 1, abort_flag, status)) {
             ok = false;
             break;
           }
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(GemmRoles<NA, BN>::kThreads, 1)
               // K steps wholly past K multiply TMA's zero fill: skip them
               if (kk > 0 && kb * KB + kk * (KB / KK) >= K) break;
               // 32 bytes of K per MMA (8 tf32 or 16 fp16): advance the start address by 2 (16-byte units)
+              if (!elect_one()) continue;
               if constexpr (CG == 2) {
                 mma_f16_pair(d, da_hi + 2 * kk, db_hi + 2 * kk, idesc, (!first || kk > 0) ? 1u : 0u);
                 if (NSPLIT == 3) {
@@ -343,19 +346,17 @@ __global__ void __launch_bounds__(GemmRoles<NA, BN>::kThreads, 1)
               }
             }
           }
-          if constexpr (CG == 2) {
-            mma_commit_pair(&empty[s]);
-            if (last) {
-              mma_commit_pair(&cfull[buf]);
-              ++c;
-            }
-          } else {
-            mma_commit(&empty[s]);
-            if (last) {
-              mma_commit(&cfull[buf]);
-              ++c;
+          if (elect_one()) {
+            if constexpr (CG == 2) {
+              mma_commit_pair(&empty[s]);
+              if (last) mma_commit_pair(&cfull[buf]);
+            } else {
+              mma_commit(&empty[s]);
+              if (last) mma_commit(&cfull[buf]);
             }
           }
+          __syncwarp();
+          if (last) ++c;
         }
       }
     }
