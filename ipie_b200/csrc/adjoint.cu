@@ -380,11 +380,11 @@ __global__ void __launch_bounds__(kVjpThreads, 1)
     energy_vjp_kernel(const double* __restrict__ rchol, const double2* __restrict__ ghalf,
                       const double2* __restrict__ rh1, const double2* __restrict__ xv, const double2* __restrict__ ebar,
                       int X, int M, int N, double f1, double fc2, double fx2, double2* __restrict__ gbar) {
-  extern __shared__ double vjp_smem[];
+  extern __shared__ __align__(16) double vjp_smem[];
   const int NM = N * M, w = blockIdx.x;
   double2* g = reinterpret_cast<double2*>(vjp_smem);  // (N, M)
-  double* l = vjp_smem + 2 * NM;                      // (N, M)
-  double2* t = reinterpret_cast<double2*>(l + NM);    // (N, N)
+  double2* t = g + NM;                                // (N, N)
+  double* l = reinterpret_cast<double*>(t + N * N);   // (N, M), last: N M may be odd
   const double2* gw = ghalf + (size_t)w * NM;
   for (int e = threadIdx.x; e < NM; e += kVjpThreads) g[e] = gw[e];
   double2 acc[kVjpPer];

@@ -226,3 +226,29 @@ def test_local_energy_vjp_tile_edges(M, na, nb, X, W):
     want = torch.autograd.grad((c * _torch_energy(ham, trial, ga, gb, False)).real.sum(), (ga, gb))
     for a, b in zip(got, want):
         assert rel(a, b) < 1e-10
+
+
+@pytest.mark.parametrize("M,na,nb,X,W", [(41, 33, 31, 5, 3),  # past N = 32 (scalar) beside the tensor cores, odd N M
+                                         (60, 40, 34, 4, 2), (181, 45, 1, 3, 2), (257, 1, 3, 4, 5), (259, 31, 7, 2, 2),
+                                         (512, 16, 1, 3, 2)])
+def test_local_energy_vjp_scalar_kernel(M, na, nb, X, W):
+    """Both sides of the N = 32 and M = 256 rules, with N M odd (the scalar kernel's arrays of unequal element
+    size share one allocation); the entry point itself, since the energy stops at N = 32.  Sums of
+    products in FP64, 1e-10 relative as above."""
+    from types import SimpleNamespace
+
+    from ipie_b200._lib import call, ptr, stream
+
+    rng = np.random.default_rng(M + na)
+    c128 = lambda *s: torch.from_numpy(rng.normal(size=s) + 1j * rng.normal(size=s)).cuda()
+    real = lambda *s: torch.from_numpy(rng.normal(size=s)).cuda()
+    ham = SimpleNamespace(nchol=X, nbasis=M, ecore=1.5)
+    trial = SimpleNamespace(_rchola=real(X, na * M), _rcholb=real(X, nb * M), _rH1a=c128(na, M), _rH1b=c128(nb, M))
+    ga, gb, c = c128(W, na, M).requires_grad_(True), c128(W, nb, M).requires_grad_(True), c128(W)
+    want = torch.autograd.grad((c * _torch_energy(ham, trial, ga, gb, False)).real.sum(), (ga, gb))
+    got = [torch.full_like(g.detach(), float("nan")) for g in (ga, gb)]
+    work = torch.empty(W * X, dtype=torch.complex128, device="cuda")
+    call("ipie_b200_local_energy_vjp", 0, ptr(trial._rchola), ptr(trial._rcholb), ptr(trial._rH1a), ptr(trial._rH1b),
+         ptr(ga.detach()), ptr(gb.detach()), W, X, M, na, nb, ptr(c), ptr(work), ptr(got[0]), ptr(got[1]), stream())
+    for a, b in zip(got, want):
+        assert rel(a.conj().resolve_conj(), b.resolve_conj()) < 1e-10  # the gradient of Re(c E) is conj(c dE/dG)
