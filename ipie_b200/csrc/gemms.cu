@@ -240,10 +240,14 @@ cudaError_t launch_taylor(const double2* vhs, const double2* phi_in, double2* ph
 // A tile takes as many whole vectors x and walkers w as fit its BM rows and BN columns, so no row or
 // column is spent on rounding N up (N = 10 in 16 x 16 blocks did 2.6 times the work); the tile shape
 // is the one of two that N fills better.  The epilogue parks T in shared memory and sums each
-// (x, w) block's products over unordered pairs (i, j) into one partial per (tile row, walker); T
-// never reaches global memory.  At 2 CTAs per SM one's epilogue runs under the other's products.
-// UHF, 640 walkers, M = 108, N = 15, X = 600, one spin: 1.99 -> 1.67 ms (37.3 GFLOP: 22
-// TFLOP/s, 25 with the padding of 15 to 120 / 8 rows); 512 walkers, M = 76, N = 10, X = 400: 0.78 -> 0.34 ms.
+// walker's products over x and the unordered pairs (i, j) into one partial per (tile row, walker); T
+// never reaches global memory.  Its terms are dealt to the lanes one by one, with the places of T_ij
+// and T_ji from a table: a warp per (x, w) block left it 512 blocks in a row with one lane at work at N = 1
+// (31 walkers, M = 20, X = 150: 167 -> 7.9 us; 64, M = 26, X = 120, N = 5: 13.5 -> 7.5 us) and divided by N
+// for every term.  At 2 CTAs per SM one's epilogue runs under the other's products.
+// UHF, 640 walkers, M = 108, N = 15, X = 600, one spin: 1.99 -> 1.56 ms (37.3 GFLOP: 24
+// TFLOP/s, 27 with the padding of 15 to 120 / 8 rows); 512 walkers, M = 76, N = 10, X = 400: 0.77 -> 0.30 ms,
+// against N rounded up to 8, 16 or 32.
 // ---------------------------------------------------------------------------
 using ExWide = RcCfg<128, 32, 4, 2, 2>;
 using ExTall = RcCfg<96, 48, 4, 2, 2>;
@@ -257,6 +261,17 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int wm0 = (warp / C::WARPS_N) * C::WTM, wn0 = (warp % C::WARPS_N) * C::WTN;
   const int x0 = (int)blockIdx.y * XB, w0 = (int)blockIdx.x * WB;
+  constexpr int NW = C::THREADS / 32, MAXN = 32;
+  __shared__ double2 red[C::BN][NW];
+  // unordered pairs of {0 .. N-1} as (i, i + d mod N), d = 0 .. N/2 (half of the last d when N is
+  // even): the places of T_ij and T_ji within a block
+  __shared__ unsigned place[MAXN * (MAXN + 1) / 2];
+  const int pairs = N * (N + 1) / 2;
+  for (int e = tid; e < pairs; e += C::THREADS) {
+    const int d = e / N, i = e - d * N, j = i + d < N ? i + d : i + d - N;
+    place[e] = (unsigned)(i * LDC + j) | (unsigned)(j * LDC + i) << 16;
+  }
+  for (int e = tid; e < WB * NW; e += C::THREADS) red[e / NW][e % NW] = make_double2(0.0, 0.0);
   RcAcc<C> acc;
   rc_mainloop<C, true, false>(X * N, W * N, x0 * N, w0 * N, op, 0, op.chunks, rc_sm, acc);
   cp_async_wait<0>();
@@ -271,31 +286,37 @@ __global__ void __launch_bounds__(C::THREADS, C::OCC)
       d[1] = make_double2(acc.re[i][j][1], acc.im[i][j][1]);
     }
   __syncthreads();
-  // unordered pairs of {0..N-1} as (i, i + d mod N), d = 0 .. N/2: once each, except that d = N/2
-  // of an even N meets every pair twice.  A warp takes consecutive (w, x) blocks, so it crosses few
-  // walkers and reduces once per walker it meets.
-  constexpr int NW = C::THREADS / 32;
-  __shared__ double2 red[C::BN][NW];
-  const int xn = min(XB, X - x0), wn = min(WB, W - w0), pairs = (N / 2 + 1) * N;
-  for (int e = tid; e < wn * NW; e += C::THREADS) red[e / NW][e % NW] = make_double2(0.0, 0.0);
-  __syncthreads();
-  const int b0 = xn * wn * warp / NW, b1 = xn * wn * (warp + 1) / NW;
-  double2 s = make_double2(0.0, 0.0);
-  for (int b = b0; b < b1; ++b) {
-    const int wl = b / xn, xl = b - wl * xn;
-    const double2* blk = sT + xl * N * LDC + wl * N;
-    for (int e = lane; e < pairs; e += 32) {
-      const int d = e / N, i = e - d * N, j = i + d < N ? i + d : i + d - N;
-      const double2 p = cmul(blk[i * LDC + j], blk[j * LDC + i]);
-      const double f = (d == 0 || 2 * d == N) ? 1.0 : 2.0;
-      s.x += f * p.x;
-      s.y += f * p.y;
+  // The (x, pair) terms of the tile, walker by walker, in equal shares per warp: the lanes take
+  // consecutive terms, whatever N is, and a warp reduces once per walker it meets.
+  const int xn = min(XB, X - x0), wn = min(WB, W - w0), terms = xn * pairs;
+  const int dx = 32 / pairs, dp = 32 - dx * pairs;
+  int e0 = wn * terms * warp / NW;
+  const int e1 = wn * terms * (warp + 1) / NW;
+  int wl = e0 / terms, q = e0 - wl * terms;
+  while (e0 < e1) {
+    const int qe = min(terms, q + e1 - e0);
+    const int first = q + lane;
+    int xl = first / pairs, p = first - xl * pairs;
+    double2 s = make_double2(0.0, 0.0);
+    for (int e = first; e < qe; e += 32) {
+      const double2* blk = sT + xl * N * LDC + wl * N;
+      const unsigned ij = place[p];
+      const double2 v = cmul(blk[ij & 0xffffu], blk[ij >> 16]);
+      const double f = p < N ? 1.0 : 2.0;
+      s.x += f * v.x;
+      s.y += f * v.y;
+      xl += dx;
+      p += dp;
+      if (p >= pairs) {
+        p -= pairs;
+        ++xl;
+      }
     }
-    if (b + 1 == b1 || xl == xn - 1) {
-      s = warp_sum2(s);
-      if (lane == 0) red[wl][warp] = s;
-      s = make_double2(0.0, 0.0);
-    }
+    s = warp_sum2(s);
+    if (lane == 0) red[wl][warp] = s;
+    e0 += qe - q;
+    q = 0;
+    ++wl;
   }
   __syncthreads();
   if (tid < wn) {

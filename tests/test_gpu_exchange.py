@@ -26,3 +26,28 @@ def test_exchange(W, X, M, N):
     want = torch.einsum("wxij,wxji->w", t, t)
     scale = (t.abs() ** 2).sum(dim=(1, 2, 3))
     assert float(((part.sum(0) - want).abs() / scale).max()) < 1e-12
+
+
+@pytest.mark.parametrize("W,X,M", [(31, 150, 20), (64, 120, 26), (256, 60, 20)])
+def test_few_electrons_cost_no_more_than_eight(W, X, M):
+    """One to five electrons are 1/64 to 1/3 of the work of eight on the same walkers and vectors, however the
+    packed tiles divide it.  A factor of two is left for launch overhead and for fewer, fuller tiles."""
+    from ipie_b200._lib import call, lib, ptr, stream
+
+    def us(N):
+        r, g = (torch.rand(n, dtype=torch.float64, device="cuda") for n in (X * N * M, 2 * W * N * M))
+        part = torch.empty(lib().ipie_b200_exchange_rows(W, X, M, N) * W * 2, dtype=torch.float64, device="cuda")
+        best = float("inf")
+        for _ in range(8):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            for _ in range(20):
+                call("ipie_b200_exchange", ptr(r), ptr(g), W, X, M, N, ptr(part), stream())
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]) * 50.0)
+        return best
+
+    eight = us(8)
+    for N in (1, 2, 3, 5):
+        assert us(N) < 2.0 * eight, N
