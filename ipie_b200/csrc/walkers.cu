@@ -343,11 +343,13 @@ __global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restr
 }
 
 // The same shift without the (X, W) transposed copy: four warps per walker (two walkers per
-// block) walk its row of vbias / xi with coalesced loads, two neighbouring fields per lane, write the
+// block) walk its row of vbias / xi with coalesced loads, V neighbouring fields per lane, write the
 // binary16 split xs_hi / xs_lo (the fields x kFieldScaleF16 as planar (W, 2, ldx) head/remainder, the
-// right operand of the mixed VHS product) in pairs and reduce cmf, cfb with shuffles and shared
-// memory (one warp per walker left ~14 warps per SM, too few to cover the loads' latency).
+// right operand of the mixed VHS product) and reduce cmf, cfb with shuffles and shared
+// memory (one warp per walker left ~14 warps per SM, too few to cover the loads' latency).  V = 2
+// stores pairs, which needs both planes on 4-byte boundaries.
 constexpr int kShiftWarps = 4;  // warps per walker
+template <int V>
 __global__ void __launch_bounds__(256) field_shift_rows_kernel(const double2* __restrict__ vbias,
                                                                const double* __restrict__ xi,
                                                                const double2* __restrict__ mf, int W, int X,
@@ -360,15 +362,15 @@ __global__ void __launch_bounds__(256) field_shift_rows_kernel(const double2* __
   const bool live = w < W;
   const int ldx = f16_ld(X);
   double2 acc_mf = make_double2(0.0, 0.0), acc_fb = make_double2(0.0, 0.0);
-  for (int x = 2 * (sub * 32 + lane); live && x < X; x += 64 * kShiftWarps) {
+  for (int x = V * (sub * 32 + lane); live && x < X; x += V * 32 * kShiftWarps) {
     const size_t e = (size_t)w * X + x;
-    const bool two = x + 1 < X;
+    const bool two = V == 2 && x + 1 < X;
     double2 xs[2];
     xs[0] = shift_one(vbias[e], mf[x], xi[e], sqrt_dt, bound, near2, acc_mf, acc_fb);
     xs[1] = make_double2(0.0, 0.0);
     if (two) xs[1] = shift_one(vbias[e + 1], mf[x + 1], xi[e + 1], sqrt_dt, bound, near2, acc_mf, acc_fb);
     if (xs_hi != nullptr) {
-      // rows of ldx (a multiple of 8) and even x: 4-byte stores; a pair's second half past X is padding
+      // (a pair starts at an even x of a row of ldx, a multiple of 8; its second half past X is padding)
       const size_t o = (size_t)w * 2 * ldx + x;
       split_store_f16(xs_hi, xs_lo, o, xs[0].x, xs[1].x, two);
       split_store_f16(xs_hi, xs_lo, o + ldx, xs[0].y, xs[1].y, two);
@@ -397,8 +399,10 @@ cudaError_t launch_field_shift(const double2* vbias, const double* xi, const dou
   // below this square |xbar| is certainly not over the bound
   const double near2 = bound > 0.0 ? bound * bound * (1.0 - 1e-12) : 0.0;
   if (xshifted == nullptr) {
-    field_shift_rows_kernel<<<(W + 1) / 2, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, near2, cmf, cfb,
-                                                         static_cast<__half*>(xs_hi), static_cast<__half*>(xs_lo));
+    const bool pairs = ((reinterpret_cast<uintptr_t>(xs_hi) | reinterpret_cast<uintptr_t>(xs_lo)) & 3) == 0;
+    auto k = pairs ? field_shift_rows_kernel<2> : field_shift_rows_kernel<1>;
+    k<<<(W + 1) / 2, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, near2, cmf, cfb, static_cast<__half*>(xs_hi),
+                                   static_cast<__half*>(xs_lo));
     note_launch();
     return cudaGetLastError();
   }
