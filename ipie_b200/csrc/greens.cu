@@ -427,15 +427,17 @@ cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M
 // tensor cores (N padded to NT tiles of 8):
 //   S = phi^H phi (lower tiles): chunks of 8 rows of phi through a cp.async ring;
 //   S = L L^H (L = R^H) and W = L^-1 in panels of 8 columns: one warp factors the panel with a row
-//       per lane (shuffles, no barriers) and inverts its diagonal block D = L_KK^-1, then all warps
-//       apply it as 8 x 8 x 8 products, three barriers per panel:
-//         W[K, J] <- D W[K, J] (J < K),  S[I, J] -= L[I, K] L[J, K]^H (I >= J > K),
-//         W[I, J] -= L[I, K] W[K, J] (I > K, J <= K).
+//       per lane (shuffles, no barriers) and solves L_KK x = (rows K of W) with a column per lane,
+//       then all warps apply them as 8 x 8 x 8 products, two barriers per panel:
+//         S[I, J] -= L[I, K] L[J, K]^H (I >= J > K),  W[I, J] -= L[I, K] W[K, J] (I > K, J <= K).
 //       W replaces S tile by tile in sm.O (column block J of S is spent once panel J is factored);
 //   phi <- phi W^H in place, chunks of 32 rows, a row tile per warp, the zero tiles of W skipped.
+// The two halves of a complex product's real and imaginary parts are summed in chains of their own.
+// That and the solves keep the rounding of plain sums: orbitals 2.7e-16 and det R 1.3e-15 off at M =
+// 200, N = 32 (joint chains and explicit inverses of the L_KK: 3.8e-16 and 1.8e-15).
 // log det R = sum log L_kk.  Its error is that of the Gram matrix, ~cond(phi)^2 eps: walkers are
 // reorthogonalised every few steps, so phi stays close to orthonormal and cond(phi) near 1.
-// 2048 walkers, M = 200, N = 32: 537 -> 291 us (419 MB of orbitals in and out: 63 us; the products' floor is
+// 2048 walkers, M = 200, N = 32: 537 -> 288 us (419 MB of orbitals in and out: 63 us; the products' floor is
 // 100 us); 512, M = 76, N = 10: 72 -> 20 us (against DFMA products, a barrier pair per Cholesky column and
 // a serial triangular inverse).
 template <int NT>
@@ -449,7 +451,7 @@ struct RoShape {
   static constexpr int CSTAGE = kChunk * LDC, XSTAGE = XM * LDX;
   static constexpr int XRING = NT == 4 ? 2 : 3;  // (two keep four walkers of 32 electrons on an SM)
   static constexpr int STAGE = RING * CSTAGE > XRING * XSTAGE ? RING * CSTAGE : XRING * XSTAGE;
-  static_assert(STAGE >= (NP + 8) * LDP, "the panel and its diagonal inverse live in the rings' room");
+  static_assert(STAGE >= NP * LDP, "the panel lives in the rings' room");
   static constexpr int UNITS = NT * (NT + 1) / 2, PER = (UNITS + WARPS - 1) / WARPS;  // lower tiles, per warp
 };
 
@@ -458,11 +460,8 @@ struct RoShared {
   using S = RoShape<NT>;
   double2 O[S::NP * S::LDO];
   union {
-    double2 stage[S::STAGE];  // copy rings of the two products with phi
-    struct {                  // between them
-      double2 P[S::NP * S::LDP];
-      double2 D[8 * S::LDP];
-    };
+    double2 stage[S::STAGE];    // copy rings of the two products with phi
+    double2 P[S::NP * S::LDP];  // between them
   };
   double diag[32];
   double spread, logsum;
@@ -474,12 +473,13 @@ __device__ __forceinline__ void lower_tile(int u, int& I, int& J) {
   J = u - I * (I + 1) / 2;
 }
 
-// (re, im) of one 8 x 8 tile += a b over 4 columns of k
-__device__ __forceinline__ void cmma(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+// one 8 x 8 tile += a b over 4 columns of k, the two halves of the real and of the imaginary part apart
+__device__ __forceinline__ void cmma(double (&re)[2], double (&im)[2], double (&re2)[2], double (&im2)[2], double2 a,
+                                     double2 b) {
   dmma884(re, a.x, b.x);
   dmma884(im, a.x, b.y);
-  dmma884(re, -a.y, b.y);
-  dmma884(im, a.y, b.x);
+  dmma884(re2, -a.y, b.y);
+  dmma884(im2, a.y, b.x);
 }
 __device__ __forceinline__ double2 conj_(double2 z) { return make_double2(z.x, -z.y); }
 
@@ -502,11 +502,13 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
       }
       cp_async_commit();
     };
-    double re[S::PER][2], im[S::PER][2];
+    // (the products of the two real and of the two mixed parts are summed apart: one chain of 2 M terms
+    // rounds 1.4 times as often)
+    double re[S::PER][2], im[S::PER][2], re2[S::PER][2], im2[S::PER][2];
     int arow[S::PER], bcol[S::PER];
 #pragma unroll
     for (int q = 0; q < S::PER; ++q) {
-      re[q][0] = re[q][1] = im[q][0] = im[q][1] = 0.0;
+      re[q][0] = re[q][1] = im[q][0] = im[q][1] = re2[q][0] = re2[q][1] = im2[q][0] = im2[q][1] = 0.0;
       int I, J;
       lower_tile(min(warp + q * S::WARPS, S::UNITS - 1), I, J);
       arow[q] = t * S::LDC + 8 * I + g;
@@ -524,7 +526,7 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
 #pragma unroll
         for (int q = 0; q < S::PER; ++q) {
           if (warp + q * S::WARPS >= S::UNITS) break;
-          cmma(re[q], im[q], conj_(st[arow[q] + kk * S::LDC]), st[bcol[q] + kk * S::LDC]);
+          cmma(re[q], im[q], re2[q], im2[q], conj_(st[arow[q] + kk * S::LDC]), st[bcol[q] + kk * S::LDC]);
         }
     }
     cp_async_wait<0>();
@@ -536,7 +538,7 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
       // S[j, i] = conj(S[i, j]): with rows I and columns J of phi^H phi this is the lower tile
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        sm.O[(8 * I + g) * S::LDO + 8 * J + 2 * t + h] = make_double2(re[q][h], im[q][h]);
+        sm.O[(8 * I + g) * S::LDO + 8 * J + 2 * t + h] = make_double2(re[q][h] + re2[q][h], im[q][h] + im2[q][h]);
     }
   }
   __syncthreads();
@@ -571,74 +573,43 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm.P[lane * S::LDP + j] = a[j];
       __syncwarp();
-      // D = L_KK^-1: lane c solves column c by forward substitution
-      if (lane < 8) {
+      // rows K of W: lane c solves L_KK x = (rows K of column c) by forward substitution
+      if (lane < 8 * kb + 8) {
         double2 x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          double2 acc = make_double2(i == lane ? 1.0 : 0.0, 0.0);
+          double2* o = sm.O + (8 * kb + i) * S::LDO + lane;
+          double2 acc = lane < 8 * kb ? *o : make_double2(i == lane - 8 * kb ? 1.0 : 0.0, 0.0);
 #pragma unroll
           for (int p = 0; p < i; ++p) acc = csub(acc, cmul(sm.P[(8 * kb + i) * S::LDP + p], x[p]));
           const double d = sm.P[(8 * kb + i) * S::LDP + i].x;
           x[i] = d != 0.0 ? make_double2(acc.x / d, acc.y / d) : make_double2(0.0, 0.0);
-          sm.D[i * S::LDP + lane] = x[i];
+          *o = x[i];
         }
       }
     }
     __syncthreads();
-    // W[K, J] <- D W[K, J] (J < K), W[K, K] = D;  S[I, J] -= L[I, K] L[J, K]^H (I >= J > K)
+    // S[I, J] -= L[I, K] L[J, K]^H (I >= J > K), W[I, J] -= L[I, K] W[K, J] (I > K >= J; W[I, K] was zero)
     for (int u = warp; u < S::UNITS; u += S::WARPS) {
       int I, J;
       lower_tile(u, I, J);
-      double2* c = sm.O + (8 * I + g) * S::LDO + 8 * J + 2 * t;
-      if (I == kb) {
-        double2 v0, v1;
-        if (J == kb) {
-          v0 = sm.D[g * S::LDP + 2 * t];
-          v1 = sm.D[g * S::LDP + 2 * t + 1];
-        } else {
-          double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
-#pragma unroll
-          for (int h = 0; h < 8; h += 4)
-            cmma(re, im, sm.D[g * S::LDP + h + t], sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g]);
-          v0 = make_double2(re[0], im[0]);
-          v1 = make_double2(re[1], im[1]);
-        }
-        __syncwarp();  // the tile is read by the warp that rewrites it
-        c[0] = v0;
-        c[1] = v1;
-      } else if (J > kb) {
-        const double2 c0 = c[0], c1 = c[1];
-        double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y};
-#pragma unroll
-        for (int h = 0; h < 8; h += 4) {
-          const double2 l = sm.P[(8 * I + g) * S::LDP + h + t];
-          cmma(re, im, make_double2(-l.x, -l.y), conj_(sm.P[(8 * J + g) * S::LDP + h + t]));
-        }
-        c[0] = make_double2(re[0], im[0]);
-        c[1] = make_double2(re[1], im[1]);
-      }
-    }
-    __syncthreads();
-    // W[I, J] -= L[I, K] W[K, J] (I > K, J <= K; W[I, K] was zero)
-    for (int u = warp; u < S::UNITS; u += S::WARPS) {
-      int I, J;
-      lower_tile(u, I, J);
-      if (I <= kb || J > kb) continue;
+      if (I <= kb) continue;
       double2* c = sm.O + (8 * I + g) * S::LDO + 8 * J + 2 * t;
       double2 c0 = make_double2(0.0, 0.0), c1 = c0;
-      if (J < kb) {
+      if (J != kb) {
         c0 = c[0];
         c1 = c[1];
       }
-      double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y};
+      double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
 #pragma unroll
       for (int h = 0; h < 8; h += 4) {
         const double2 l = sm.P[(8 * I + g) * S::LDP + h + t];
-        cmma(re, im, make_double2(-l.x, -l.y), sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g]);
+        const double2 r = J > kb ? conj_(sm.P[(8 * J + g) * S::LDP + h + t])
+                                 : sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g];
+        cmma(re, im, re2, im2, make_double2(-l.x, -l.y), r);
       }
-      c[0] = make_double2(re[0], im[0]);
-      c[1] = make_double2(re[1], im[1]);
+      c[0] = make_double2(re[0] + re2[0], im[0] + im2[0]);
+      c[1] = make_double2(re[1] + re2[1], im[1] + im2[1]);
     }
     __syncthreads();
   }
@@ -691,14 +662,14 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
     for (int k = 0; k < 2 * NT; ++k) av[k] = a[4 * k];
 #pragma unroll
     for (int J = 0; J < NT; ++J) {
-      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
       const double2* w = sm.O + (8 * J + col) * S::LDO + t;
 #pragma unroll
-      for (int k = 0; k < 2 * (J + 1); ++k) cmma(re, im, av[k], conj_(w[4 * k]));
+      for (int k = 0; k < 2 * (J + 1); ++k) cmma(re, im, re2, im2, av[k], conj_(w[4 * k]));
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const int j = 8 * J + 4 * q + t;
-        if (m < M && j < N) phi[(size_t)m * N + j] = make_double2(re[q], im[q]);
+        if (m < M && j < N) phi[(size_t)m * N + j] = make_double2(re[q] + re2[q], im[q] + im2[q]);
       }
     }
   }

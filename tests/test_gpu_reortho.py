@@ -57,3 +57,42 @@ def test_reortho_matches_householder(M, N, cond, tol):
         assert abs(np.log(detR[w].item()) - logdet) < 1e-10 * max(1.0, abs(logdet))
         assert abs(logd[w].item() - logdet) < 1e-10 * max(1.0, abs(logdet))
         assert abs(ovlp[w].item() - np.exp(-logdet)) < 1e-10 * abs(np.exp(-logdet))
+
+
+def _gram_schmidt(phi):
+    """Q and log det R in extended precision (Gram-Schmidt with a second sweep)."""
+    a = phi.astype(np.clongdouble)
+    q, ld = np.zeros_like(a), np.zeros(len(a), dtype=np.longdouble)
+    for j in range(a.shape[2]):
+        v = a[:, :, j].copy()
+        for _ in range(2):
+            c = np.einsum("wmk,wm->wk", q[:, :, :j].conj(), v)
+            v = v - np.einsum("wmk,wk->wm", q[:, :, :j], c)
+        r = np.sqrt((np.abs(v) ** 2).sum(1))
+        ld += np.log(r)
+        q[:, :, j] = v / r[:, None]
+    return q, ld
+
+
+@pytest.mark.parametrize("M,N,W,most_q,most_det", [(200, 32, 48, 3.2e-16, 1.65e-15), (76, 10, 96, 2.0e-16, 5.6e-16),
+                                                  (120, 24, 48, 2.75e-16, 1.2e-15)])
+def test_reortho_rounding(M, N, W, most_q, most_det):
+    """Rounding on walkers as a walk leaves them (cond near 1), rms over the batch.  The bounds are about 1.15
+    times what sums of M terms with triangular solves show; sums of 2 M terms (both halves of a complex
+    product in one chain) or an explicit inverse of R's diagonal blocks show 1.3 to 1.4 times."""
+    from ipie_b200._lib import call, ptr, stream
+
+    rng = np.random.default_rng(1)
+    psi = np.linalg.qr(rng.normal(size=(M, N)))[0]
+    phi0 = psi + 0.3 / M ** 0.5 * (rng.normal(size=(W, M, N)) + 1j * rng.normal(size=(W, M, N)))
+    want, ld = _gram_schmidt(phi0)
+    phi = torch.from_numpy(phi0).cuda()
+    shift, det, logd = (torch.zeros(W, dtype=torch.float64, device="cuda") for _ in range(3))
+    ovlp = torch.ones(W, dtype=torch.complex128, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("ipie_b200_reortho", ptr(phi), ptr(phi), W, M, N, 0, ptr(shift), ptr(det), ptr(logd), ptr(ovlp), ptr(status),
+         stream())
+    assert int(status.item()) == 0
+    q, d = phi.cpu().numpy(), det.cpu().numpy().astype(np.longdouble)
+    assert float(np.linalg.norm((q - want).ravel()) / np.linalg.norm(want.ravel())) < most_q
+    assert float(np.sqrt(np.mean((d / np.exp(ld) - 1) ** 2))) < most_det
