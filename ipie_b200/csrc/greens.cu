@@ -24,6 +24,9 @@ constexpr int kChunk = 8;  // rows of phi / psi* per shared-memory chunk of the 
 //         A[:, J] <- A[:, J] (pivot rows zeroed) + panel' A[pivot rows, J].
 //       So a column costs no barrier and a panel three, where the column by column form took two
 //       per column.
+//       The halves of a complex product are summed apart, here and in O, and an entry takes a panel's
+//       products in one addition: Ghalf 4.3e-16 and the overlap 1.6e-15 off at M = 200, N = 32, complex trial
+//       (6.9e-16 and 3.5e-15 with every product added to the entries in turn).
 //   With p_k the pivot row of column k the stored array B holds O^-1[k, p_j] = B[p_k, j].
 //   Ghalf[i, m] = sum_c O^-1[i, c] phi[m, c]: warp w keeps its rows of O^-1 as MMA fragments in
 //       registers (gathered through p once) while chunks of 16 rows of phi pass through the ring.
@@ -31,10 +34,10 @@ constexpr int kChunk = 8;  // rows of phi / psi* per shared-memory chunk of the 
 //       lanes store four neighbouring entries of Ghalf; rows of an odd stride keep the fragment
 //       loads free of bank conflicts.
 // The floor is the f64 tensor pipe's time for the two products (28k cycles per SM and walker at
-// M = 200, N = 32).  2048 walkers, M = 200, N = 32: 535 -> 354 us; 512, M = 76, N = 10: 46 -> 19 us; 777, M =
+// M = 200, N = 32).  2048 walkers, M = 200, N = 32: 535 -> 324 us; 512, M = 76, N = 10: 46 -> 19 us; 777, M =
 // 149, N = 23 + 17: 280 -> 175 us (against DFMA products and the column by column elimination), and 175 ->
 // 151 us with a CTA per spin instead of both in one (640, M = 108, N = 15 + 15: 89 -> 72 us): the pivot chains of
-// the two spins run side by side and the last round of CTAs is shorter.
+// the two spins run side by side and the last round of CTAs is shorter (144 us with the sums above).
 template <int NT>
 struct GfShape {
   static constexpr int WARPS = NT == 3 ? 3 : 4, THREADS = 32 * WARPS, NP = 8 * NT;
@@ -83,9 +86,11 @@ __device__ __forceinline__ void gf_overlap_tiles(const double2* __restrict__ phi
   };
   constexpr int CT = NT >= 3 ? NT : 1;  // column tiles per warp
   const int rt = NT >= 3 ? warp : NT == 2 ? (warp & 1) : 0, ct0 = NT == 2 ? (warp >> 1) : 0;
-  double re[CT][2], im[CT][2];
+  // (the halves of a complex product in chains of their own: one chain of 2 M terms rounds more)
+  double re[CT][2], im[CT][2], re2[CT][2], im2[CT][2];
 #pragma unroll
-  for (int j = 0; j < CT; ++j) re[j][0] = re[j][1] = im[j][0] = im[j][1] = 0.0;
+  for (int j = 0; j < CT; ++j)
+    re[j][0] = re[j][1] = im[j][0] = im[j][1] = re2[j][0] = re2[j][1] = im2[j][0] = im2[j][1] = 0.0;
   issue(0);
   issue(1);
   for (int ch = 0; ch < nch; ++ch) {
@@ -105,12 +110,19 @@ __device__ __forceinline__ void gf_overlap_tiles(const double2* __restrict__ phi
         const double2 bv = b[kk * S::LDC + 8 * j];
         dmma884(re[j], av.x, bv.x);
         dmma884(im[j], av.x, bv.y);
-        dmma884(re[j], -av.y, bv.y);
-        dmma884(im[j], av.y, bv.x);
+        dmma884(re2[j], -av.y, bv.y);
+        dmma884(im2[j], av.y, bv.x);
       }
     }
   }
   cp_async_wait<0>();
+#pragma unroll
+  for (int j = 0; j < CT; ++j)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      re[j][q] += re2[j][q];
+      im[j][q] += im2[j][q];
+    }
   if (NT == 1) {
     __syncthreads();  // the ring is free: the four partial tiles
     double2* part = sm.stage + warp * 64 + g * 8 + 2 * t;
@@ -223,25 +235,23 @@ __device__ __forceinline__ void gf_invert(int N, GfShared<NT>& sm, unsigned* sta
 #pragma unroll
     for (int j = 0; j < CT; ++j) {
       if (ct0 + j == kb) continue;
-      double2* c = sm.O + row * S::LDO + 8 * (ct0 + j) + 2 * t;
-      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
-      if (!pivot) {
-        const double2 c0 = c[0], c1 = c[1];
-        re[0] = c0.x;
-        re[1] = c1.x;
-        im[0] = c0.y;
-        im[1] = c1.y;
+      // the products summed by themselves, their halves apart: small beside the entries they change, so
+      // that an entry is rounded once a panel and not with every term
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 a = h == 0 ? a0 : a1;
+        dmma884(re, a.x, b[j][h].x);
+        dmma884(im, a.x, b[j][h].y);
+        dmma884(re2, -a.y, b[j][h].y);
+        dmma884(im2, a.y, b[j][h].x);
       }
-      dmma884(re, a0.x, b[j][0].x);
-      dmma884(im, a0.x, b[j][0].y);
-      dmma884(re, -a0.y, b[j][0].y);
-      dmma884(im, a0.y, b[j][0].x);
-      dmma884(re, a1.x, b[j][1].x);
-      dmma884(im, a1.x, b[j][1].y);
-      dmma884(re, -a1.y, b[j][1].y);
-      dmma884(im, a1.y, b[j][1].x);
-      c[0] = make_double2(re[0], im[0]);
-      c[1] = make_double2(re[1], im[1]);
+      double2* c = sm.O + row * S::LDO + 8 * (ct0 + j) + 2 * t;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double2 v = make_double2(re[q] + re2[q], im[q] + im2[q]);
+        c[q] = pivot ? v : cadd(c[q], v);
+      }
     }
     __syncthreads();
   }

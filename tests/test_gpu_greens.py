@@ -69,3 +69,43 @@ def test_singular_overlap_is_flagged():
     assert int(status.item()) & 2
     want, det = _reference(pa[::2], q)
     assert float((g[::2] - want).norm() / want.norm()) < 1e-10  # the other walkers are unharmed
+
+
+def _extended(phi, psi_conj):
+    """Ghalf (W, N, M) and det O in extended precision: elimination, and an FP64 inverse refined."""
+    p = phi.astype(np.clongdouble)
+    o = np.einsum("wmi,mj->wij", p, psi_conj.astype(np.clongdouble))
+    a, det, w = o.copy(), np.ones(len(o), dtype=np.clongdouble), np.arange(len(o))
+    for k in range(o.shape[1]):
+        r = k + np.argmax(np.abs(a[:, k:, k]), axis=1)
+        t = a[w, r].copy()
+        a[w, r] = a[:, k]
+        a[:, k] = t
+        det *= np.where(r != k, -1, 1) * a[:, k, k]
+        a[:, k + 1:, k:] -= (a[:, k + 1:, k] / a[:, k, k][:, None])[:, :, None] * a[:, None, k, k:]
+    x, one = np.linalg.inv(o.astype(complex)).astype(np.clongdouble), np.eye(o.shape[1])
+    for _ in range(3):
+        x = x + np.einsum("wij,wjk->wik", x, one - np.einsum("wij,wjk->wik", o, x))
+    return np.einsum("wij,wmj->wim", x, p), det
+
+
+@pytest.mark.parametrize("M,N,W,most_g,most_o", [(200, 32, 48, 5.4e-16, 2.5e-15), (76, 10, 96, 3.4e-16, 8.5e-16)])
+def test_greens_rounding(M, N, W, most_g, most_o):
+    """Rounding for a complex trial and walkers near it, rms over the batch.  The bounds are about 1.2 times what
+    O's sums of M terms and one rounding of an entry per panel show; both halves of a complex product in
+    one chain, of 2 M terms and on the entries themselves, show 1.3 to 2 times."""
+    from ipie_b200._lib import call, ptr, stream
+
+    rng = np.random.default_rng(1)
+    psi = np.linalg.qr(rng.normal(size=(M, N)) + 1j * rng.normal(size=(M, N)))[0]
+    phi = psi + 0.3 / M ** 0.5 * (rng.normal(size=(W, M, N)) + 1j * rng.normal(size=(W, M, N)))
+    psi_conj = np.ascontiguousarray(psi.conj())
+    want, det = _extended(phi, psi_conj)
+    p, q = torch.from_numpy(phi).cuda(), torch.from_numpy(psi_conj).cuda()
+    g, ov = torch.empty(W, N, M, dtype=p.dtype, device="cuda"), torch.empty(W, dtype=p.dtype, device="cuda")
+    ls, status = torch.zeros(W, dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("ipie_b200_greens_function_single_det_batch", ptr(p), ptr(p), W, M, N, 0, ptr(q), ptr(q), ptr(ls), ptr(g),
+         ptr(g), ptr(ov), None, ptr(status), stream())
+    assert int(status.item()) == 0
+    assert float(np.linalg.norm((g.cpu().numpy() - want).ravel()) / np.linalg.norm(want.ravel())) < most_g
+    assert float(np.sqrt(np.mean(np.abs(ov.cpu().numpy() / det - 1) ** 2))) < most_o
