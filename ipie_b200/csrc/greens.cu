@@ -19,8 +19,9 @@ constexpr int kChunk = 8;  // rows of phi / psi* per shared-memory chunk of the 
 //       owns row tile w of O (NT = 1: a quarter of the rows m, NT = 2: one of the four tiles).
 //   O^-1 by Gauss-Jordan elimination in place, partial pivoting on |.|, in panels of 8 columns: one
 //       warp factors the panel with a row per lane and the 8 columns in registers (the pivot by one
-//       redux.sync on the float bits of |a|^2 above the row index, its row by shuffles; pivots stay
-//       in their rows), then all warps apply it to the other columns as one rank-8 MMA update
+//       redux.sync on the high word of |a|^2 above the row index, so one within 2^-15 of the largest
+//       |a|^2; its row by shuffles; pivots stay in their rows), then all warps apply it to the other
+//       columns as one rank-8 MMA update
 //         A[:, J] <- A[:, J] (pivot rows zeroed) + panel' A[pivot rows, J].
 //       So a column costs no barrier and a panel three, where the column by column form took two
 //       per column.
@@ -172,7 +173,7 @@ __device__ __forceinline__ void gf_invert(int N, GfShared<NT>& sm, unsigned* sta
           unsigned key = 0u;
           const double2 own = a[jj];
           if (lane < N && !((used >> lane) & 1u))
-            key = (__float_as_uint((float)cabs2(own)) & ~31u) | (unsigned)(31 - lane);
+            key = ((unsigned)__double2hiint(cabs2(own)) & ~31u) | (unsigned)(31 - lane);
           // every lane scales its row as if it held the pivot, while the pivot is found
           const double rn = __drcp_rn(own.x * own.x + own.y * own.y);
           const double2 pinv = make_double2(own.x * rn, -own.y * rn);
@@ -182,7 +183,8 @@ __device__ __forceinline__ void gf_invert(int N, GfShared<NT>& sm, unsigned* sta
           key = __reduce_max_sync(0xffffffffu, key);
           int p = 31 - (int)(key & 31u);
           if (key < 32u) {
-            // no positive |a|^2 left (an exactly singular block, or NaN): any free row
+            // every free |a|^2 is zero (an exactly singular block, or |a| below 1e-154): any free row.  A
+            // NaN has a large key and is taken.
             p = __ffs(~used) - 1;
           }
           const bool mine = lane == p;

@@ -71,6 +71,31 @@ def test_singular_overlap_is_flagged():
     assert float((g[::2] - want).norm() / want.norm()) < 1e-10  # the other walkers are unharmed
 
 
+@pytest.mark.parametrize("N", [5, 10, 19, 32])
+@pytest.mark.parametrize("scale", [1e-25, 1e-100, 1e60])
+def test_pivot_of_a_scaled_column(N, scale):
+    """A column of O far from 1 whose first entry is zero: the pivot is still the column's largest entry."""
+    from ipie_b200._lib import call, ptr, stream
+
+    M, W = 40, 3
+    rng = np.random.default_rng(N)
+    cplx = lambda *s: torch.from_numpy(rng.normal(size=s) + 1j * rng.normal(size=s)).cuda()
+    pa, q = cplx(W, M, N), cplx(M, N)
+    pa[:, : M // 2, 0] = 0  # O[0, 0] = 0
+    q[M // 2:, 0] = 0
+    q[:, 0] *= scale
+    ls = torch.zeros(W, dtype=torch.float64, device="cuda")
+    g, ov = torch.empty(W, N, M, dtype=pa.dtype, device="cuda"), torch.empty(W, dtype=pa.dtype, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("ipie_b200_greens_function_single_det_batch", ptr(pa), ptr(pa), W, M, N, 0, ptr(q), ptr(q), ptr(ls), ptr(g),
+         ptr(g), ptr(ov), None, ptr(status), stream())
+    assert int(status.item()) == 0
+    want, det = _reference(pa, q)
+    err = (g - want).abs().amax(dim=(0, 2)) / want.abs().amax(dim=(0, 2))  # row by row: row 0 carries 1 / scale
+    assert float(err.max()) < 1e-10
+    assert float(((ov - det).abs() / det.abs()).max()) < 1e-10
+
+
 def _extended(phi, psi_conj):
     """Ghalf (W, N, M) and det O in extended precision: elimination, and an FP64 inverse refined."""
     p = phi.astype(np.clongdouble)
