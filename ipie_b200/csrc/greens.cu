@@ -356,11 +356,11 @@ __global__ void __launch_bounds__(GfShape<NT>::THREADS, 4)
   extern __shared__ __align__(16) unsigned char gf_sm[];
   GfShared<NT>& sm = *reinterpret_cast<GfShared<NT>*>(gf_sm);
   // two distinct spin blocks: a cluster of two CTAs, one per spin (S = 2); one block, or one
-  // counted twice (phib == phia with nb == na): one CTA
+  // counted twice (phib == phia with nb == na): one CTA.  (na >= 1: the launchers refuse less)
   const int w = blockIdx.x / S, s = blockIdx.x % S;
-  const bool alias = S == 1 && nb > 0 && na > 0;
-  const int N = S == 2 ? (s == 0 ? na : nb) : max(na, nb);
-  const bool beta = S == 2 ? s == 1 : na == 0;
+  const bool alias = S == 1 && nb > 0;
+  const int N = s == 0 ? na : nb;
+  const bool beta = s == 1;
   const double2* phi = (beta ? phib : phia) + (size_t)w * M * N;
   gf_overlap_tiles<NT>(phi, beta ? psib_c : psia_c, M, N, sm);
   __syncthreads();
@@ -422,7 +422,7 @@ cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M
   auto k = ghalfa != nullptr ? gf_mma_kernel<NT, true> : gf_mma_kernel<NT, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  const int S = na > 0 && nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
+  const int S = nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   spin_config(cfg, attr, W, S, GfShape<NT>::THREADS, smem, st);
@@ -703,9 +703,9 @@ __global__ void __launch_bounds__(RoShape<NT>::THREADS, 4)
   RoShared<NT>& sm = *reinterpret_cast<RoShared<NT>*>(gf_sm);
   // as the Green's function: one CTA per distinct spin block, a walker's two in a cluster
   const int w = blockIdx.x / S, s = blockIdx.x % S;
-  const bool alias = S == 1 && nb > 0 && na > 0;
-  const int N = S == 2 ? (s == 0 ? na : nb) : max(na, nb);
-  double2* phi = ((S == 2 ? s == 1 : na == 0) ? phib : phia) + (size_t)w * M * N;
+  const bool alias = S == 1 && nb > 0;
+  const int N = s == 0 ? na : nb;
+  double2* phi = (s == 0 ? phia : phib) + (size_t)w * M * N;
   double l = cholqr_block<NT>(phi, M, N, sm, status);
   // CholQR2: a second pass over the (now nearly orthonormal) result when R's diagonal spreads
   // by more than kCholQR2 (the first pass's error grows like cond(phi)^2 eps); R = R2 R1, so
@@ -738,7 +738,7 @@ cudaError_t launch_reortho_nt(double2* phia, double2* phib, int W, int M, int na
   auto k = reortho_chol32_kernel<NT>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  const int S = na > 0 && nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
+  const int S = nb > 0 && !(phib == phia && nb == na) ? 2 : 1;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
   spin_config(cfg, attr, W, S, RoShape<NT>::THREADS, smem, st);
