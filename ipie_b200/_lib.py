@@ -72,6 +72,7 @@ SIGNATURES = {
     "ipie_b200_energy_complex": [P, P, I, I, I, P, P, D, P, P, I, P, P, P],
     "ipie_b200_exchange_complex": [P, P, I, I, I, I, P, P, I, P],
     "ipie_b200_umma_gemm_f16_test": [P, P, P, P, P, I, I, I, I, P, P],
+    "ipie_b200_rc_plan_test": [I, I, I, P, P],
     "ipie_b200_normal_fill": [P, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_ulonglong, P],
     "ipie_b200_normal_fill_dev": [P, ctypes.c_longlong, ctypes.c_ulonglong, P, P],
     "ipie_b200_pair_branch": [I, P, P, D, D, D, ctypes.c_ulonglong, P, I, P, P, P, P, P, P],

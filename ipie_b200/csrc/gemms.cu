@@ -1,6 +1,7 @@
 // GEMM-shaped stages of the FP64 walker step on the f64 tensor cores
 // (DMMA): force bias, VHS assembly, one-body propagation, the Taylor series
 // of exp(VHS), and the fused exchange energy.
+#include "../../include/ipie_b200_testing.h"
 #include "gemm_f64.cuh"
 #include "gemm_rc.cuh"
 #include "kernels.h"
@@ -376,3 +377,10 @@ cudaError_t launch_exchange(const double* rchol, const double2* ghalf, int W, in
 }
 
 }  // namespace ipie_b200
+
+extern "C" int ipie_b200_rc_plan_test(int M, int N, int chunks, int* tile, int* split) {
+  const ipie_b200::RcPlan p = ipie_b200::rc_plan(M, N, chunks);
+  *tile = p.tile;
+  *split = p.S;
+  return 0;
+}
