@@ -18,7 +18,8 @@
 // Small outputs leave most SMs idle and make K a serial chain (a 120 x 64 output is two 128 x 32
 // tiles), so the tile shape and a split of K over a cluster of S CTAs are chosen together from the
 // sizes (rc_plan): the S partial tiles are added through distributed shared memory in rank order,
-// which needs no workspace and keeps the result the same from run to run.
+// which needs no workspace and keeps the result the same from run to run (for one batch size: another
+// one can take another split and so add a walker's terms in another order).
 //
 // The bound is the f64 tensor pipe (36.9 TFLOP/s with operands in registers).  Measured, with two
 // register-staged 128 x 64 tiles and one launch per operand before: force bias of 1024 walkers,
