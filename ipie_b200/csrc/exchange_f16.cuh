@@ -1,5 +1,6 @@
 // Exchange of the mixed-precision energy with the walkers' Green's functions held in tensor memory
-// (M <= 256; longer K rows take umma_gemm_kernel<EpiExchange>):
+// (M <= 256 and more than a tile or two per SM, see exchange_streams in mixed.cu; the rest takes
+// umma_gemm_kernel<EpiExchange>):
 //
 //     raw_w = sum_x sum_ij T_ij T_ji,      T = L_x G_w^T (N x N complex),
 //

@@ -1058,7 +1058,7 @@ static cudaError_t device_sms(int* sms) {
 
 template <int NP>
 static cudaError_t exchange_tmem_np(const void* r_hi, const void* r_lo, double rscale, const GPad& gp, int W, int X,
-                                    int M, double2* part, unsigned* status, cudaStream_t st) {
+                                    int M, int sms, double2* part, unsigned* status, cudaStream_t st) {
   using S = ExTmemShape;
   const int Mp = f16_ld(M);
   if (W <= 0 || X <= 0) return cudaErrorInvalidValue;
@@ -1069,8 +1069,6 @@ static cudaError_t exchange_tmem_np(const void* r_hi, const void* r_lo, double r
   if ((e = map_f16_pair(&maps.b_hi, &maps.b_lo, r_hi, r_lo, (long long)X * NP, M, Mp, S::BN, false, &maps.b_planes)) !=
       cudaSuccess)
     return e;
-  int sms = 0;
-  if ((e = device_sms(&sms)) != cudaSuccess) return e;
   auto kern = exchange_tmem_kernel<NP>;
   if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES)) != cudaSuccess)
     return e;
@@ -1081,17 +1079,39 @@ static cudaError_t exchange_tmem_np(const void* r_hi, const void* r_lo, double r
   return cudaGetLastError();
 }
 
-// The walkers' rows stay in tensor memory up to M = 256 (two planes of 128 columns next to the two
-// accumulator buffers); longer rows stream both operands.
+// Whether both operands stream.  The walkers' rows stay in tensor memory up to M = 256 (two planes of 128
+// columns next to the two accumulator buffers), except where a CTA has one tile, or two of which the second
+// needs other rows: loading the rows, a thread per row, is then as long as a tile and nothing hides it.
+// Measured, tensor memory and streamed: 4 walkers, M = 224, N = 12, X = 672 (84 tiles): 24.3 and 22.6 us; 12
+// walkers, M = 200, N = 12, X = 600 (225 tiles, runs across walker tiles): 33.0 and 28.0; 8 walkers (150, none
+// across): 25.3 and 27.0; 24 (375): 33.9 and 42.5; below the two M the rows are short enough: 96 walkers, M =
+// 120, N = 3, X = 360 (276 tiles, across): 20.4 and 23.0.
+static bool exchange_streams(int W, int X, int M, int NP, int sms) {
+  if (M > ExTmemShape::MAX_K) return true;
+  if (M <= (NP == 8 ? 160 : 120)) return false;
+  const ExRuns runs = exchange_tmem_runs(W, X, NP, sms);
+  const long long tiles = (long long)runs.nwt * runs.nxt;
+  if (tiles <= sms || tiles > 2LL * sms) return tiles <= sms;
+  for (int i = 1; i < runs.nwt % runs.g; ++i) {
+    const long long t = (long long)i * runs.nxt;
+    if (runs.first(runs.run_of(t)) != t) return true;
+  }
+  return false;
+}
+
 static cudaError_t exchange3(const void* r_hi, const void* r_lo, double rscale, const GPad& gp, int W, int X, int M,
                              int N, double2* part, unsigned* status, cudaStream_t st) {
-  if (M <= ExTmemShape::MAX_K) switch (exchange_np(N)) {
-      case 8: return exchange_tmem_np<8>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
-      case 16: return exchange_tmem_np<16>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
-      case 32: return exchange_tmem_np<32>(r_hi, r_lo, rscale, gp, W, X, M, part, status, st);
+  const int np = exchange_np(N);
+  int sms = 0;
+  const cudaError_t e = device_sms(&sms);
+  if (e != cudaSuccess) return e;
+  if (!exchange_streams(W, X, M, np, sms)) switch (np) {
+      case 8: return exchange_tmem_np<8>(r_hi, r_lo, rscale, gp, W, X, M, sms, part, status, st);
+      case 16: return exchange_tmem_np<16>(r_hi, r_lo, rscale, gp, W, X, M, sms, part, status, st);
+      case 32: return exchange_tmem_np<32>(r_hi, r_lo, rscale, gp, W, X, M, sms, part, status, st);
       default: return cudaErrorInvalidValue;
     }
-  switch (exchange_np(N)) {
+  switch (np) {
     case 8: return exchange3_np<8>(r_hi, r_lo, rscale, gp, W, X, M, N, part, status, st);
     case 16: return exchange3_np<16>(r_hi, r_lo, rscale, gp, W, X, M, N, part, status, st);
     case 32: return exchange3_np<32>(r_hi, r_lo, rscale, gp, W, X, M, N, part, status, st);
@@ -1103,7 +1123,8 @@ static cudaError_t exchange3(const void* r_hi, const void* r_lo, double rscale, 
 static int exchange3_rows(int W, int X, int M, int N) {
   const int np = exchange_np(N);
   int sms = 0;
-  if (M <= ExTmemShape::MAX_K && device_sms(&sms) == cudaSuccess) return exchange_tmem_runs(W, X, np, sms).rows();
+  if (device_sms(&sms) == cudaSuccess && !exchange_streams(W, X, M, np, sms))
+    return exchange_tmem_runs(W, X, np, sms).rows();
   return (X * np + kBM - 1) / kBM;
 }
 

@@ -1,5 +1,5 @@
-"""The mixed exchange with the Green's function in tensor memory (M <= 256) and beside it (M > 256): runs that
-split a walker tile, several walker tiles per run, K steps that end inside a chunk, every row padding;
+"""The mixed exchange with the Green's function in tensor memory (M <= 256) and streamed (M > 256, and longer rows on
+one or two tiles per SM): runs that split a walker tile, several walker tiles per run, K steps that end inside a chunk, every row padding;
 against torch in complex128.  Each product carries ~3 x 2^-22 from the split operands and ~2^-17 x K / 2048
 at most from FP32 accumulation over chunks of 128 K; relative to sum |T_ij|^2 that stays below 3e-6."""
 import numpy as np
@@ -12,7 +12,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("W,X,M,N", [(1, 1, 4, 1), (3, 5, 26, 5), (17, 333, 65, 8), (9, 41, 64, 9), (300, 23, 133, 15),
                                      (5, 700, 128, 16), (1, 601, 129, 17), (301, 7, 200, 23), (33, 150, 256, 32),
-                                     (7, 30, 257, 12), (4, 9, 264, 32)])
+                                     (7, 30, 257, 12), (4, 9, 264, 32),
+                                     # streamed for few tiles, for runs across walker tiles; neither; short rows
+                                     (4, 100, 224, 12), (12, 600, 200, 12), (8, 600, 200, 12), (12, 600, 120, 12)])
 def test_exchange_mixed(W, X, M, N):
     from ipie_b200._lib import call, ptr, stream
 
