@@ -444,9 +444,10 @@ cudaError_t launch_gf_mma(const double2* phia, const double2* phib, int W, int M
 //         S[I, J] -= L[I, K] L[J, K]^H (I >= J > K),  W[I, J] -= L[I, K] W[K, J] (I > K, J <= K).
 //       W replaces S tile by tile in sm.O (column block J of S is spent once panel J is factored);
 //   phi <- phi W^H in place, chunks of 32 rows, a row tile per warp, the zero tiles of W skipped.
-// The two halves of a complex product's real and imaginary parts are summed in chains of their own.
-// That and the solves keep the rounding of plain sums: orbitals 2.7e-16 and det R 1.3e-15 off at M =
-// 200, N = 32 (joint chains and explicit inverses of the L_KK: 3.8e-16 and 1.8e-15).
+// The halves of a complex product of the Gram matrix are summed in chains of their own, a panel's products by
+// themselves before they change an entry, and phi W^H with its largest terms last.  That and the solves keep
+// the rounding of plain sums: orbitals 2.5e-16 and det R 1.25e-15 off at M = 200, N = 32 (joint chains, every
+// product added to the entry in turn and explicit inverses of the L_KK: 3.8e-16 and 1.8e-15).
 // log det R = sum log L_kk.  Its error is that of the Gram matrix, ~cond(phi)^2 eps: walkers are
 // reorthogonalised every few steps, so phi stays close to orthonormal and cond(phi) near 1.
 // 2048 walkers, M = 200, N = 32: 537 -> 288 us (419 MB of orbitals in and out: 63 us; the products' floor is
@@ -485,13 +486,13 @@ __device__ __forceinline__ void lower_tile(int u, int& I, int& J) {
   J = u - I * (I + 1) / 2;
 }
 
-// one 8 x 8 tile += a b over 4 columns of k, the two halves of the real and of the imaginary part apart
-__device__ __forceinline__ void cmma(double (&re)[2], double (&im)[2], double (&re2)[2], double (&im2)[2], double2 a,
-                                     double2 b) {
-  dmma884(re, a.x, b.x);
+// (re, im) of one 8 x 8 tile += a b over 4 columns of k; the products with b's real part last, which hold
+// the large terms where b is near a real diagonal
+__device__ __forceinline__ void cmma(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+  dmma884(re, -a.y, b.y);
   dmma884(im, a.x, b.y);
-  dmma884(re2, -a.y, b.y);
-  dmma884(im2, a.y, b.x);
+  dmma884(re, a.x, b.x);
+  dmma884(im, a.y, b.x);
 }
 __device__ __forceinline__ double2 conj_(double2 z) { return make_double2(z.x, -z.y); }
 
@@ -538,7 +539,11 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
 #pragma unroll
         for (int q = 0; q < S::PER; ++q) {
           if (warp + q * S::WARPS >= S::UNITS) break;
-          cmma(re[q], im[q], re2[q], im2[q], conj_(st[arow[q] + kk * S::LDC]), st[bcol[q] + kk * S::LDC]);
+          const double2 a = st[arow[q] + kk * S::LDC], b = st[bcol[q] + kk * S::LDC];
+          dmma884(re[q], a.x, b.x);
+          dmma884(im[q], a.x, b.y);
+          dmma884(re2[q], a.y, b.y);
+          dmma884(im2[q], -a.y, b.x);
         }
     }
     cp_async_wait<0>();
@@ -607,21 +612,17 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
       lower_tile(u, I, J);
       if (I <= kb) continue;
       double2* c = sm.O + (8 * I + g) * S::LDO + 8 * J + 2 * t;
-      double2 c0 = make_double2(0.0, 0.0), c1 = c0;
-      if (J != kb) {
-        c0 = c[0];
-        c1 = c[1];
-      }
-      double re[2] = {c0.x, c1.x}, im[2] = {c0.y, c1.y}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
 #pragma unroll
       for (int h = 0; h < 8; h += 4) {
         const double2 l = sm.P[(8 * I + g) * S::LDP + h + t];
         const double2 r = J > kb ? conj_(sm.P[(8 * J + g) * S::LDP + h + t])
                                  : sm.O[(8 * kb + h + t) * S::LDO + 8 * J + g];
-        cmma(re, im, re2, im2, make_double2(-l.x, -l.y), r);
+        cmma(re, im, l, r);
       }
-      c[0] = make_double2(re[0] + re2[0], im[0] + im2[0]);
-      c[1] = make_double2(re[1] + re2[1], im[1] + im2[1]);
+      // (the products summed by themselves, then one rounding of the entry)
+      c[0] = J == kb ? make_double2(-re[0], -im[0]) : make_double2(c[0].x - re[0], c[0].y - im[0]);
+      c[1] = J == kb ? make_double2(-re[1], -im[1]) : make_double2(c[1].x - re[1], c[1].y - im[1]);
     }
     __syncthreads();
   }
@@ -674,14 +675,14 @@ __device__ __noinline__ double cholqr_block(double2* __restrict__ phi, int M, in
     for (int k = 0; k < 2 * NT; ++k) av[k] = a[4 * k];
 #pragma unroll
     for (int J = 0; J < NT; ++J) {
-      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0}, re2[2] = {0.0, 0.0}, im2[2] = {0.0, 0.0};
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
       const double2* w = sm.O + (8 * J + col) * S::LDO + t;
 #pragma unroll
-      for (int k = 0; k < 2 * (J + 1); ++k) cmma(re, im, re2, im2, av[k], conj_(w[4 * k]));
+      for (int k = 0; k < 2 * (J + 1); ++k) cmma(re, im, av[k], conj_(w[4 * k]));
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const int j = 8 * J + 4 * q + t;
-        if (m < M && j < N) phi[(size_t)m * N + j] = make_double2(re[q] + re2[q], im[q] + im2[q]);
+        if (m < M && j < N) phi[(size_t)m * N + j] = make_double2(re[q], im[q]);
       }
     }
   }
