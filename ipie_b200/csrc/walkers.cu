@@ -278,8 +278,8 @@ __device__ __forceinline__ double2 shift_one(double2 v, double2 m, double r, dou
 // that both sides move whole 128-byte lines.  The share is one of a cluster's S (the host's choice:
 // about four CTAs per SM, 64 fields or more each), whose partial sums are added through distributed
 // shared memory in rank order.  The first version, one CTA per 32 walkers over all of X, ran 2 to 32
-// CTAs: 84 -> 13.5 us at 640 walkers, X = 600; 37 -> 5.4 us at 256 walkers, X = 320; 14.7 -> 3.6 us at 64
-// walkers, X = 120.
+// CTAs.  Replayed from a graph: 50 -> 10.6 us at 640 walkers, X = 600; 27 -> 4.9 us at 256 walkers, X =
+// 320; 12 -> 3.7 us at 64 walkers, X = 120.
 constexpr int kShiftWalkers = 8, kShiftStep = 64;
 __global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restrict__ vbias,
                                                           const double* __restrict__ xi,
@@ -347,7 +347,9 @@ __global__ void __launch_bounds__(256) field_shift_kernel(const double2* __restr
 // binary16 split xs_hi / xs_lo (the fields x kFieldScaleF16 as planar (W, 2, ldx) head/remainder, the
 // right operand of the mixed VHS product) and reduce cmf, cfb with shuffles and shared
 // memory (one warp per walker left ~14 warps per SM, too few to cover the loads' latency).  V = 2
-// stores pairs, which needs both planes on 4-byte boundaries.
+// stores pairs, which needs both planes on 4-byte boundaries, and is taken above 64 fields, which one warp's
+// pairs would leave to two fields in a row (640 walkers, replayed from a graph, V = 1 and 2: X = 64: 2.46 and
+// 2.66 us; X = 128: 2.95 and 2.78; X = 512: 4.31 and 4.11; 2048 walkers, X = 1600: 23.7 and 20.4).
 constexpr int kShiftWarps = 4;  // warps per walker
 template <int V>
 __global__ void __launch_bounds__(256) field_shift_rows_kernel(const double2* __restrict__ vbias,
@@ -399,7 +401,8 @@ cudaError_t launch_field_shift(const double2* vbias, const double* xi, const dou
   // below this square |xbar| is certainly not over the bound
   const double near2 = bound > 0.0 ? bound * bound * (1.0 - 1e-12) : 0.0;
   if (xshifted == nullptr) {
-    const bool pairs = ((reinterpret_cast<uintptr_t>(xs_hi) | reinterpret_cast<uintptr_t>(xs_lo)) & 3) == 0;
+    const bool pairs = X > 64 &&
+                       ((reinterpret_cast<uintptr_t>(xs_hi) | reinterpret_cast<uintptr_t>(xs_lo)) & 3) == 0;
     auto k = pairs ? field_shift_rows_kernel<2> : field_shift_rows_kernel<1>;
     k<<<(W + 1) / 2, 256, 0, st>>>(vbias, xi, mf, W, X, sqrt_dt, bound, near2, cmf, cfb, static_cast<__half*>(xs_hi),
                                    static_cast<__half*>(xs_lo));
