@@ -525,12 +525,12 @@ __device__ __forceinline__ uint32_t split2_f16(float y0, float y1, uint32_t& lo)
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// The epilogue goes through shared memory and TMA tensor stores: two 32 KB staging boxes of 64
+// The epilogue goes through shared memory and TMA tensor stores: 32 KB staging boxes of 64
 // walkers x 16 rows x 16 halves (the {16, 16, 64} box of the plane maps maps->out: re_hi, re_lo,
-// im_hi, im_lo), one for the real plane (filled by the rows c = 1) and one for the imaginary (c = 0),
-// filled and stored four times per tile -- the transposed block (J, I) then the block (I, J), head
-// then remainder.  (One box, eight times, kept half the threads idle: 24.7 -> 21.1 us at 512 walkers,
-// M = 76, 116 -> 104 us at 700 walkers, M = 132; equal at 2048 walkers, M = 200, 1.14 ms.)  A thread's
+// im_hi, im_lo), the real plane's filled by the rows c = 1 and the imaginary's by the rows c = 0.
+// BOXES = 2: both at once, filled and stored four times per tile -- the transposed block (J, I) then
+// the block (I, J), head then remainder.  BOXES = 1: one box, eight times, the real plane first; half the
+// threads wait, and the ring has room for a fourth stage (vhs_one_box says when).  A thread's
 // scattered 16-byte global stores (one 32-byte sector
 // split between two of them, 16 walkers per warp instruction) took ~30k cycles per tile and
 // stalled the next tile's products; the staged tensor stores leave the copy to the TMA engine.
@@ -541,12 +541,14 @@ __device__ __forceinline__ uint32_t split2_f16(float y0, float y1, uint32_t& lo)
 // (k = (lane / 2) mod 8) writes its chunks in an order rotated by k instead: its block chunks
 // (8 rows x two 16-byte halves) rotated by k within each half of eight, which spreads the lanes
 // over all 32 banks (four wavefronts per instruction of 512 bytes), and the transposed rows b rotated by
-// k mod 4 within each group of four (a transposed row has one 16-byte half per column group).  The values are split into head and remainder once per tile.
+// k mod 4 within each group of four (a transposed row has one 16-byte half per column group).  The
+// values are split into head and remainder once per tile.
+template <int BOXES>
 struct EpiVHSBlock {
   int M, W, nb;  // nb: 16-orbital blocks per side
   float f;       // sqrt(dt) v_scale / (operand scales)
   static constexpr int kBox = 64 * 16 * 32;
-  static constexpr int kSmemBytes = 2 * kBox;
+  static constexpr int kSmemBytes = BOXES * kBox;
   static constexpr bool kUsesMaps = true;
   static constexpr int kThreads = 256;  // the epilogue threads of the 128 x 256 tile (barrier 3)
   __device__ __forceinline__ static void sync() { asm volatile("bar.sync 3, %0;\n" ::"r"(kThreads) : "memory"); }
@@ -608,35 +610,39 @@ struct EpiVHSBlock {
     const int g = (col0 >> 7) & 1;
     const float s = c ? -f : f;
     const int k = (threadIdx.x >> 1) & 7;
-    // the rows c = 1 feed the real plane, c = 0 the imaginary one: one box each per round
-    uint8_t* mine = smem + (1 - c) * kBox + wl * 512;
+    uint8_t* mine = smem + (BOXES == 2 ? (1 - c) * kBox : 0) + wl * 512;
     // head / remainder pairs: word 8 a + m holds columns 2m, 2m + 1 of the thread's row a
     uint32_t ph[64], pl[64];
 #pragma unroll
     for (int e = 0; e < 64; ++e) ph[e] = split2_f16(v[2 * e] * s, v[2 * e + 1] * s, pl[e]);
 #pragma unroll
-    for (int rd = 0; rd < 4; ++rd) {
-      const int tr = rd < 2, lo = rd & 1;
-      if (tr && I == J) continue;  // the same for every thread of the tile
-      if (rd == 2) {
-        rotate(ph, k);
-        rotate(pl, k);
-      }
-      if (threadIdx.x == 0) bulk_wait_read_all();  // the previous boxes have left shared memory
-      sync();
-      if (live) {
-        if (lo)
-          put(pl, tr, k, g, mine);
-        else
-          put(ph, tr, k, g, mine);
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      }
-      sync();
-      if (threadIdx.x == 0) {
+    for (int pass = 0; pass < 2 / BOXES; ++pass) {
+      const bool act = live && (BOXES == 2 || c == 1 - pass);
 #pragma unroll
-        for (int pc = 0; pc < 2; ++pc)
-          tma_store_3d(&maps->out[2 * pc + lo], tr ? 16 * I : 16 * J, tr ? 16 * J : 16 * I, w0, smem + pc * kBox);
-        bulk_commit();
+      for (int rd = 0; rd < 4; ++rd) {
+        const int tr = rd < 2, lo = rd & 1;
+        if (tr && I == J) continue;  // the same for every thread of the tile
+        if (rd == 2 && (BOXES == 2 || act)) {
+          rotate(ph, k);
+          rotate(pl, k);
+        }
+        if (threadIdx.x == 0) bulk_wait_read_all();  // the previous boxes have left shared memory
+        sync();
+        if (act) {
+          if (lo)
+            put(pl, tr, k, g, mine);
+          else
+            put(ph, tr, k, g, mine);
+          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
+        sync();
+        if (threadIdx.x == 0) {
+#pragma unroll
+          for (int pc = 0; pc < BOXES; ++pc)
+            tma_store_3d(&maps->out[2 * (pass + pc) + lo], tr ? 16 * I : 16 * J, tr ? 16 * J : 16 * I, w0,
+                         smem + pc * kBox);
+          bulk_commit();
+        }
       }
     }
   }
@@ -1161,6 +1167,14 @@ int vhs_blocks(int M) {
   return nb * (nb + 1) / 2;
 }
 
+// One staging box and four ring stages, or two and three.  Two are the faster (24.5 and 20.9 us at 512
+// walkers, M = 76, X = 400; 110 and 99 at 700, M = 132, X = 524) except where the rows of a plane end in half a
+// 32-byte sector and the planes are larger than L2: a tile's neighbour completes the sectors later, and with
+// both planes under way at once more of them leave L2 in between (1.01 and 1.08 ms at 2048 walkers, M = 200,
+// X = 1000; 746 and 790 us at 1500; 255 and 248 at 512, where they are 160 MB; M = 208, whole sectors: 0.79
+// and 0.77 ms at 2048).
+static bool vhs_one_box(int W, int M) { return f16_ld(M) % 16 != 0 && 8LL * W * M * f16_ld(M) > (256LL << 20); }
+
 // The block-tiled VHS (EpiVHSBlock): fields (2W, X) as the left operand, the block-tiled
 // Cholesky (vhs_blocks(M) * 256, X) as the right one, 128 x 256 tiles with the walker tiles
 // fastest so that each Cholesky block is read from DRAM once while the fields stay in L2.
@@ -1184,11 +1198,13 @@ cudaError_t mixed_vhs_blocks(const void* cb_hi, const void* cb_lo, int X, int M,
   void* planes[4] = {re_hi, re_lo, im_hi, im_lo};
   for (int p = 0; p < 4; ++p)
     if ((e = make_map_f16_store(&maps.out[p], planes[p], W, M, f16_ld(M), 16, 16, 64)) != cudaSuccess) return e;
-  const EpiVHSBlock epi{M, W, (M + 15) / 16, (float)(sqrt_dt / (cb_scale * kFieldScaleF16) * v_scale)};
-  // 64-byte K rows: three 48 KB stages (four, and two of 96 KB, ran the main loop no faster) leave
-  // room for two boxes in the epilogue
-  return launch_umma<BN, 1, 3, 3, EpiVHSBlock, KIND_F16_K32>(maps, X, 0, 0, grid, epi, status, st, true,
-                                                            persistent != 0);
+  // 64-byte K rows: three 48 KB stages next to two boxes, four next to one
+  const float f = (float)(sqrt_dt / (cb_scale * kFieldScaleF16) * v_scale);
+  if (vhs_one_box(W, M))
+    return launch_umma<BN, 1, 3, 4, EpiVHSBlock<1>, KIND_F16_K32>(maps, X, 0, 0, grid, {M, W, (M + 15) / 16, f}, status,
+                                                                  st, true, persistent != 0);
+  return launch_umma<BN, 1, 3, 3, EpiVHSBlock<2>, KIND_F16_K32>(maps, X, 0, 0, grid, {M, W, (M + 15) / 16, f}, status,
+                                                                st, true, persistent != 0);
 }
 
 // Orbital update of one spin block: phi_out = E exp(V) E phi_in (Taylor order nmax),

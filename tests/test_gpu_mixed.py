@@ -83,7 +83,9 @@ def test_mixed_vhs_3pass():
 
 
 @pytest.mark.parametrize("M,X,W,persistent", [(64, 128, 24, 0), (108, 216, 70, 1), (76, 152, 130, 0),
-                                              (200, 400, 9, 1), (200, 400, 200, 0)])
+                                              (200, 400, 9, 1), (200, 400, 200, 0),
+                                              # half-sector rows on planes larger than L2: one staging box
+                                              (200, 400, 850, 1), (196, 392, 870, 0)])
 def test_mixed_vhs_blocks(M, X, W, persistent):
     """The block-tiled VHS (16 x 16 pair blocks, fields as the left operand) writes the same
     binary16 planes as the packed-pair product, with the pad columns zero; M = 108 and 76 end on
