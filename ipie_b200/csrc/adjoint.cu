@@ -91,6 +91,15 @@ struct VjpShape {
 // smallest stride >= n that is 4 modulo m (m a power of two)
 static int stride4(int n, int m) { return n + ((4 - n) & (m - 1)); }
 
+// The split with the least time: the rounds in which the clusters run, times a CTA's blocks -- 10 per step of
+// 4 K and round of S tiles over the warps, a warp's 1 to 8 accumulator tiles per 4 K of the second product
+// (kVjTiles: odd counts check each tile, seven and eight spill), 1350 for barriers and the copy -- and 9000 for
+// start and end, 3000 more for the cluster's sum.  The units are relative; they and the clusters that run
+// at once (whole ones per group of SMs: 33 of four, 15 of eight) are fitted to 251 shapes with every split of
+// each (1 to 777 walkers, M = 26 to 250, N = 1 to 32): the choice is within 0.4 % of the best on average, 13 %
+// at worst.  31 walkers, X = 500, M = 110, N = 2: 22 us with clusters of eight, 76 with single CTAs; 31, X = 1000, M =
+// 200, N = 20: 1.25 ms with clusters of four, 2.67 of eight.
+constexpr double kVjTiles[kVjMaxUnits] = {20.0, 48.0, 87.0, 103.0, 160.0, 197.0, 248.0, 344.0};
 static bool vjp_shape(int W, int X, int M, int N, VjpShape& best) {
   if (M > 256 || N > 32) return false;
   double best_cost = 0.0;
@@ -124,10 +133,10 @@ static bool vjp_shape(int W, int X, int M, int N, VjpShape& best) {
     const int nblk = (X + s.XB - 1) / s.XB;
     for (s.S = 1; s.S <= 8; s.S *= 2) {
       if (s.S > nblk) break;
-      const long long ctas = (long long)((W + s.WB - 1) / s.WB) * s.S;
-      const double waves = (double)((ctas + 147) / 148);
-      const double block = (double)((s.RT * s.CT1 + kVjWarps - 1) / kVjWarps) * s.MP4 + s.units * s.KB4 + 60.0;
-      const double cost = waves * (block * ((nblk + s.S - 1) / s.S) + (s.S > 1 ? 4000.0 : 1000.0));
+      const int at_once = s.S == 1 ? 148 : s.S == 2 ? 74 : s.S == 4 ? 33 : 15;
+      const double rounds = (double)(((W + s.WB - 1) / s.WB + at_once - 1) / at_once);
+      const double block = 10.0 * ((s.RT * s.CT1 + kVjWarps - 1) / kVjWarps) * s.MP4 + kVjTiles[s.units - 1] * s.KB4 + 1350.0;
+      const double cost = rounds * (block * ((nblk + s.S - 1) / s.S) + (s.S > 1 ? 12000.0 : 9000.0));
       if (!found || cost < best_cost) {
         best = s;
         best_cost = cost;

@@ -202,12 +202,13 @@ def test_local_energy_vjp_central_difference():
     assert abs(ad - fd) < 1e-6 * max(1.0, abs(fd))
 
 
-@pytest.mark.parametrize("M,na,nb,X,W", [(33, 7, 1, 41, 5),  # odd rows (8-byte copies)
-                                         (33, 7, 1, 400, 5),  # the same, one spin's X over a cluster of eight
+@pytest.mark.parametrize("M,na,nb,X,W", [(33, 7, 1, 41, 5),  # odd rows (8-byte copies), a cluster of four
+                                         (33, 7, 1, 400, 5),  # clusters of eight and of four
                                          (51, 9, 5, 643, 9),  # both spins' over clusters of eight, ragged shares
                                          (76, 10, 9, 50, 301),  # several walkers per CTA, a ragged last one
                                          (200, 32, 31, 9, 3),  # one Cholesky vector per block, full shared memory, clusters
-                                         (256, 32, 32, 5, 2),  # single-buffered
+                                         (256, 32, 32, 5, 2),  # single-buffered, clusters of four
+                                         (60, 9, 8, 20, 200),  # clusters of two, single CTAs
                                          (260, 8, 3, 7, 2),  # past M = 256: the scalar kernel
                                          (8, 1, 1, 1, 1)])
 def test_local_energy_vjp_tile_edges(M, na, nb, X, W):
