@@ -465,7 +465,7 @@ int ipie_b200_onebody_adjoint(int W, int M, int na, int nb, const void* ghalfa, 
  *   dE/dG_s = f1 rH1_s + 2 fc sum_x X_x L_s,x - 2 fx sum_x (L_s,x G_s^T) L_s,x,
  *   X_x = sum_s L_s,x . G_s, L_s,x row x of rchol_s as (n_s, M).
  * ebar (W) complex; work: W*X complex; out: gbara (W,na,M), gbarb (W,nb,M) complex.
- * n_s * M <= 8192; FP64 tensor cores for M <= 256, CUDA cores above. */
+ * n_s * M <= 8192; FP64 tensor cores for M <= 256 and n_s <= 32, CUDA cores beyond. */
 int ipie_b200_local_energy_vjp(int rhf, const double* rchola, const double* rcholb, const void* rH1a,
                                const void* rH1b, const void* ghalfa, const void* ghalfb, int W, int X, int M, int na,
                                int nb, const void* ebar, void* work, void* gbara, void* gbarb, void* stream);

@@ -381,7 +381,7 @@ static cudaError_t launch_vjp_mma(const double* rchol, const double2* ghalf, con
 }
 
 // Blocks the tensor-core kernel does not take (M > 256, whose G and L_x do not fit shared memory
-// together): one CTA per walker runs the sum over x with L_x, G and T_x in shared memory and the
+// together, or N > 32, more row tiles than a warp holds at large M): one CTA per walker runs the sum over x with L_x, G and T_x in shared memory and the
 // accumulator (N M complex) in registers, 16 entries per thread at most.
 constexpr int kVjpThreads = 512;
 constexpr int kVjpPer = 16;  // N * M <= 8192
