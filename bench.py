@@ -222,10 +222,10 @@ DRAM_TRAFFIC = {
     # FP16 orbital chain (transposed products) at 512 walkers: 220.1 MB read + 35.9 MB written per
     # launch (profiles/orbital_chain_t16_c2_w512.md), x4 for 2048 walkers (its traffic is per walker)
     ("c2_rhf_m200", "mixed", "orbitals"): 4 * (220.10e6 + 35.86e6),
-    # block-tiled VHS product with TMA-store epilogue at 512 walkers: 244.9 MB read + 178.5 MB
+    # block-tiled VHS product with TMA-store epilogue at 512 walkers: 236.6 MB read + 174.6 MB
     # written (profiles/vhs_blocks_tma_c2_w512.md); the Cholesky operand (~150 MB) is read once per
     # launch whatever the walker count, the fields and planes scale with it
-    ("c2_rhf_m200", "mixed", "vhs"): 4 * (244.9e6 - 150.0e6 + 178.5e6) + 150.0e6,
+    ("c2_rhf_m200", "mixed", "vhs"): 4 * (236.6e6 - 150.0e6 + 174.6e6) + 150.0e6,
 }
 
 
