@@ -1108,6 +1108,7 @@ static bool exchange_streams(int W, int X, int M, int NP, int sms) {
 static cudaError_t exchange3(const void* r_hi, const void* r_lo, double rscale, const GPad& gp, int W, int X, int M,
                              int N, double2* part, unsigned* status, cudaStream_t st) {
   const int np = exchange_np(N);
+  if (np < 0 || W <= 0 || X <= 0) return cudaErrorInvalidValue;  // (before the rule divides by tiles)
   int sms = 0;
   const cudaError_t e = device_sms(&sms);
   if (e != cudaSuccess) return e;
